@@ -44,18 +44,31 @@ __global__ void k_rows_bitrev(const cpx<T> *in, cpx<T> *out, int logh, long long
     }
 }
 
+// (grid: x over the columns, y over groups of FILL_ROWS rows, whose loads are
+// in flight together: one a thread leaves the memory idle, 3 TB/s)
+constexpr int FILL_ROWS = 8;
 template <typename T>
-__global__ void k_herm_fill(cpx<T> *out, long long H, long long W, long long ld, long long batch, long long odist)
+__global__ void __launch_bounds__(256)
+    k_herm_fill(cpx<T> *out, int logh, long long W, long long ld, long long rows, long long odist)
 {
-    const long long m = W / 2 - 1;  // columns W/2+1 .. W-1
-    const long long total = batch * H * m;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const long long col = W / 2 + 1 + idx % m;
-        const long long rest = idx / m;
-        const long long k = rest % H, b = rest / H;
-        cpx<T> *p = out + b * odist;
-        st_c(p + k * ld + col, conj(ld_c(p + ((H - k) & (H - 1)) * ld + (W - col))));
+    pdl_enter();  // launched by launch_pdl: waits for the previous kernel
+    const long long H = 1LL << logh;
+    const long long col = W / 2 + 1 + (long long)blockIdx.x * 256 + threadIdx.x;
+    if (col >= W) return;
+    // last image first: the column pass has just written it, it is in L2
+    for (long long r1 = rows - (long long)blockIdx.y * FILL_ROWS; r1 > 0; r1 -= (long long)gridDim.y * FILL_ROWS) {
+        const long long r0 = r1 - FILL_ROWS;
+        cpx<T> v[FILL_ROWS];
+#pragma unroll
+        for (int j = 0; j < FILL_ROWS; j++) {
+            const long long r = r0 + j, b = r >> logh, k = r & (H - 1);
+            if (r >= 0) v[j] = ld_c(out + b * odist + ((H - k) & (H - 1)) * ld + (W - col));
+        }
+#pragma unroll
+        for (int j = 0; j < FILL_ROWS; j++) {
+            const long long r = r0 + j, b = r >> logh, k = r & (H - 1);
+            if (r >= 0) stcs_c(out + b * odist + k * ld + col, conj(v[j]));
+        }
     }
 }
 
@@ -82,12 +95,13 @@ cudaError_t launch_rows_bitrev(int dtype, const void *in, void *out, int logh, l
 cudaError_t launch_herm_fill(int dtype, void *out, long long H, long long W, long long ld, long long batch,
                              long long odist, cudaStream_t st)
 {
-    const long long total = batch * H * (W / 2 - 1);
-    if (W < 4 || total <= 0) return cudaSuccess;
-    const unsigned g = elem_grid(total);
-    if (dtype == GFFT_F32) k_herm_fill<float><<<g, 256, 0, st>>>((cpx<float> *)out, H, W, ld, batch, odist);
-    else k_herm_fill<double><<<g, 256, 0, st>>>((cpx<double> *)out, H, W, ld, batch, odist);
-    return cudaGetLastError();
+    if (W < 4 || batch * H <= 0) return cudaSuccess;
+    const void *fn = dtype == GFFT_F32 ? (const void *)&k_herm_fill<float> : (const void *)&k_herm_fill<double>;
+    long long rows = batch * H;
+    int logh = ilog2ll(H);
+    void *args[] = {(void *)&out, (void *)&logh, (void *)&W, (void *)&ld, (void *)&rows, (void *)&odist};
+    const dim3 grid((unsigned)((W / 2 - 1 + 255) / 256), (unsigned)std::min<long long>((rows + FILL_ROWS - 1) / FILL_ROWS, 65535));
+    return launch_pdl(fn, grid, dim3(256), args, 0, st);
 }
 
 }  // namespace gfft

@@ -62,17 +62,23 @@ __device__ __forceinline__ cpx<float> operator-(cpx<float> a, cpx<float> b)
 template <typename T>
 __device__ __forceinline__ cpx<T> operator-(cpx<T> a) { return {-a.x, -a.y}; }
 
+// The products below spell out their fused multiply-adds: left to the
+// compiler, the product that is rounded first can differ from kernel to
+// kernel, and paths that promise each other's bits would not keep them.
+__device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
+
 // complex product a*b
 template <typename T>
 __device__ __forceinline__ cpx<T> cmul(cpx<T> a, cpx<T> b)
 {
-    return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x};
+    return {fma_(a.x, b.x, -(a.y * b.y)), fma_(a.x, b.y, a.y * b.x)};
 }
 // a * conj(b)
 template <typename T>
 __device__ __forceinline__ cpx<T> cmulc(cpx<T> a, cpx<T> b)
 {
-    return {a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y};
+    return {fma_(a.x, b.x, a.y * b.y), fma_(a.y, b.x, -(a.x * b.y))};
 }
 // twiddle product in the transform's direction: forward multiplies by w,
 // inverse by conj(w) (tables hold the forward twiddles exp(-2 pi i k/N)).
@@ -197,14 +203,44 @@ __device__ __forceinline__ cpx<T> rot32(cpx<T> a)
         // general root: cos(2 pi k/32), -sin(2 pi k/32); sin(t) = cos(t - pi/2)
         constexpr T wr = (T)cos32d(k);
         constexpr T wi = (T)(-cos32d(k - 8));
-        return {a.x * wr - a.y * wi, a.x * wi + a.y * wr};
+        return {fma_(a.x, wr, -(a.y * wi)), fma_(a.x, wi, a.y * wr)};
+    }
+}
+
+// Multiplication by W_64^k: the odd multiples of 2 pi / 64, else rot32.
+// Constants are the correctly rounded values of cos(pi m / 32), m odd.
+__host__ __device__ constexpr double cos64d(int k)
+{
+    k = ((k % 64) + 64) % 64;
+    if (k > 32) k = 64 - k;
+    if (k > 16) return -cos64d(32 - k);
+    return k % 2 == 0 ? cos32d(k / 2)
+         : k == 1  ? 0.99518472667219688624
+         : k == 3  ? 0.95694033573220886494
+         : k == 5  ? 0.88192126434835502971
+         : k == 7  ? 0.77301045336273696081
+         : k == 9  ? 0.63439328416364549822
+         : k == 11 ? 0.47139673682599764856
+         : k == 13 ? 0.29028467725446236764
+                   : 0.09801714032956060199;
+}
+template <int K, bool INV, typename T>
+__device__ __forceinline__ cpx<T> rot64(cpx<T> a)
+{
+    constexpr int k = INV ? ((64 - (K % 64)) % 64) : (K % 64);
+    if constexpr (k % 2 == 0) {
+        return rot32<k / 2, false, T>(a);
+    } else {
+        constexpr T wr = (T)cos64d(k);
+        constexpr T wi = (T)(-cos64d(k - 16));
+        return {fma_(a.x, wr, -(a.y * wi)), fma_(a.x, wi, a.y * wr)};
     }
 }
 
 // ---------------------------------------------------------------------------
-// In-register DFT of R points (R = 1, 2, 4, 8, 16, 32), natural order in
+// In-register DFT of R points (R = 1, 2, 4, 8, 16, 32, 64), natural order in
 // and out, stride-1 over the array v.  R >= 8 is split as A x B
-// (A = 2 for R = 8, else 4): n = n1 + A*n2, k = k1 + B*k2,
+// (A = 2 for R = 8, 8 for R = 64, else 4): n = n1 + A*n2, k = k1 + B*k2,
 //   X[k1 + B k2] = sum_n1 W_A^(n1 k2) W_R^(n1 k1) sum_n2 x[n1 + A n2] W_B^(n2 k1)
 template <int R, bool INV, typename T>
 __device__ __forceinline__ void dft(cpx<T> *v)
@@ -225,7 +261,7 @@ __device__ __forceinline__ void dft(cpx<T> *v)
         v[1] = d02 + jd13;
         v[3] = d02 - jd13;
     } else {
-        constexpr int A = (R >= 16) ? 4 : 2;
+        constexpr int A = (R == 64) ? 8 : (R >= 16) ? 4 : 2;
         constexpr int B = R / A;
         cpx<T> y[A][B];
 #pragma unroll
@@ -234,14 +270,14 @@ __device__ __forceinline__ void dft(cpx<T> *v)
             for (int n2 = 0; n2 < B; n2++) y[n1][n2] = v[n1 + A * n2];
             dft<B, INV, T>(y[n1]);
         }
-        // inner twiddles W_R^(n1 k1) = W_32^(n1 k1 32/R)
-        constexpr int S = 32 / R;
+        // inner twiddles W_R^(n1 k1) = W_64^(n1 k1 64/R)
+        constexpr int S = 64 / R;
         static_for<0, B>([&](auto k1c) {
             constexpr int k1 = decltype(k1c)::value;
             cpx<T> z[A];
             static_for<0, A>([&](auto n1c) {
                 constexpr int n1 = decltype(n1c)::value;
-                z[n1] = rot32<n1 * k1 * S, INV, T>(y[n1][k1]);
+                z[n1] = rot64<n1 * k1 * S, INV, T>(y[n1][k1]);
             });
             dft<A, INV, T>(z);
 #pragma unroll

@@ -4,10 +4,10 @@
 // Path per size (the defaults, each measured on GB300; the environment
 // knobs read below override them):
 //   C2C  n <= 2^14 (fp32) / 2^13 (fp64)  one fused kernel (c2c_fused.cu)
-//        fp32 2^16 .. 2^19               the persistent four-step kernel
+//        fp32 2^16                       the persistent four-step kernel
 //                                        (fourstep.cuh), one launch a batch
-//        fp32 2^21 .. 2^24               three passes of short tiles
-//                                        (threepass.cu) per workspace group
+//        fp32 2^17 .. 2^24               column + row launches of the
+//                                        pipelined tiles (tiles_pipe.cuh)
 //        otherwise                       column + row tile launches per
 //                                        workspace group (tiles*.cuh), the
 //                                        widest TMA-pipelined tile that fits
@@ -63,6 +63,23 @@ static void wn_tables(int dtype, int logn, int *lo_bits, const void **lo, const 
     *hi = cached_table(key + "/hi", dtype, N >> *lo_bits, fill(N >> *lo_bits, 1LL << *lo_bits));
 }
 
+// the inter-pass twiddle tables of a tiles_pipe.cuh kernel over N = 2^logn:
+// t1[e] = W_N^e for e < N / E, t2[e] = W_N^(G e) for e < N / G
+static void t12_tables(int dtype, int logn, const TileKernel *k, const void **t1, const void **t2)
+{
+    const long long N = 1LL << logn;
+    auto fill = [N](long long count, long long mul) {
+        return [N, count, mul](void *buf) {
+            for (long long e = 0; e < count; e++)
+                forward_root<float>(e * mul, N, &((float *)buf)[2 * e], &((float *)buf)[2 * e + 1]);
+        };
+    };
+    const std::string key = "t12/" + std::to_string(logn) + "/";
+    const long long n1 = N / k->e, n2 = N / k->g;
+    *t1 = cached_table(key + "1/" + std::to_string(k->e), dtype, n1, fill(n1, 1));
+    *t2 = cached_table(key + "2/" + std::to_string(k->g), dtype, n2, fill(n2, k->g));
+}
+
 static const void *tile_table(int dtype, const TileKernel *k, int logl, int c)
 {
     return cached_table("tile/" + std::to_string(dtype) + "/" + std::to_string(logl) + "/" + std::to_string(c) +
@@ -96,26 +113,32 @@ void C2CCore::init(int dtype_, int logn_, long long batch_hint, int path, bool r
     // the two-launch tile path: always set up (the persistent kernel needs
     // 16-byte aligned inputs for its tensor copies and uses it otherwise)
     const int maxc = (int)env_ll("GFFT_TILE_MAXC", 16);
-    ccol = tile_widest(dtype, TILE_COL_TW4, logA, maxc);
-    crow = tile_widest(dtype, TILE_ROW_XPOSE, logB, maxc);
+    // the pipelined tiles of 32 and 64 points a thread (tiles_pipe.cuh, which
+    // gives the measurements): fp32 2^17 and up.  At 2^16 they are faster for
+    // small batches only (one transform 9.7 us against 15.8, 2048 of them
+    // 2920 GB/s against 3056 for the persistent kernel), which stays there
+    // (GFFT_PIPE=1 / 0 overrides).  GFFT_FS, GFFT_FS_PAIR and GFFT_3PASS
+    // still name the paths they did.
+    const long long want_pipe = env_ll("GFFT_PIPE", -1);
+    const bool pipe = dtype == GFFT_F32 && path <= 0 && !real_rows && logn >= 16 &&
+                      (want_pipe > 0 || (want_pipe < 0 && logn >= 17 && env_ll("GFFT_3PASS", 0) <= 0 &&
+                                         env_ll("GFFT_FS", 0) == 0 && env_ll("GFFT_FS_PAIR", 0) == 0)) &&
+                      tile_widest(dtype, TILE_COL_TWP, logA, maxc) && tile_widest(dtype, TILE_ROW_PIPE, logB, maxc);
+    const int vcol = pipe ? TILE_COL_TWP : TILE_COL_TW4, vrow = pipe ? TILE_ROW_PIPE : TILE_ROW_XPOSE;
+    ccol = tile_widest(dtype, vcol, logA, maxc);
+    crow = tile_widest(dtype, vrow, logB, maxc);
     if (!ccol || !crow) fail(GFFT_ERR_UNSUPPORTED, "no tile kernel for this length");
-    kcol = tile_find(dtype, TILE_COL_TW4, logA, ccol);
-    krow = tile_find(dtype, TILE_ROW_XPOSE, logB, crow);
+    kcol = tile_find(dtype, vcol, logA, ccol);
+    krow = tile_find(dtype, vrow, logB, crow);
+    if (pipe) t12_tables(dtype, logn, kcol, &tw_lo, &tw_hi);
     tw_col = tile_table(dtype, kcol, logA, ccol);
     tw_row = tile_table(dtype, krow, logB, crow);
 
     // three passes of short tiles (threepass.cu), through a workspace of the
-    // tile launches' size (GFFT_3PASS=1 / 0 overrides the measured default)
+    // tile launches' size, on request (GFFT_3PASS=1)
     const ThreePass *tpk = threepass_find(dtype, logn);
-    // measured on GB300 (1 GB batches, forward + inverse, GB/s, two passes
-    // against three): 2^19 2028 / 1892, 2^20 2136 / 2067, 2^21 2006 / 2117,
-    // 2^22 1870 / 2041, 2^23 1789 / 1978, 2^24 1554 / 1934
-    const bool tp_default = logn >= 21;
-    // (an explicit request for the persistent kernels, GFFT_FS=1 or
-    // GFFT_FS_PAIR=1, keeps them)
     const long long want_tp = env_ll("GFFT_3PASS", -1);
-    const bool fs_asked = env_ll("GFFT_FS", 0) != 0 || env_ll("GFFT_FS_PAIR", 0) != 0;
-    if (tpk && path < 0 && !real_rows && (want_tp > 0 || (want_tp < 0 && tp_default && !fs_asked))) {
+    if (tpk && path < 0 && !real_rows && !pipe && want_tp > 0) {
         tp = tpk;
         for (int p = 0; p < 3; p++) {
             const int l = p == 0 ? tp->la : p == 1 ? tp->lb : tp->lc;
@@ -141,12 +164,11 @@ void C2CCore::init(int dtype_, int logn_, long long batch_hint, int path, bool r
     const bool want_pair = !real_rows && !pair_vars.empty() && env_ll("GFFT_FS_PAIR", 0) != 0;
     const FourStepKernel *const *vars = want_pair ? pair_vars.data() : plain_vars.data();
     int nvar = (int)(want_pair ? pair_vars.size() : plain_vars.size());
-    // measured on GB300 (batches of 770 transforms of 2^15 .. 2^18 points,
-    // 385 of 2^19, ...): the persistent kernel is the faster one for fp32
-    // n = 2^16 .. 2^19; the tile launches for 2^15, for 2^20 and above, and
-    // for fp64
-    const bool fs_default = dtype == GFFT_F32 && logn >= 16 && logn <= 19;
-    const bool use_fs = path >= 0 ? path == 1 : (want_pair || env_ll("GFFT_FS", fs_default ? 1 : 0) != 0);
+    // measured on GB300 (batches of 770 transforms): the persistent kernel is
+    // the faster one for fp32 n = 2^16 (2987 GB/s against 2888), the tile
+    // launches for 2^15 and for fp64
+    const bool fs_default = dtype == GFFT_F32 && logn == 16;
+    const bool use_fs = pipe ? false : path >= 0 ? path == 1 : (want_pair || env_ll("GFFT_FS", fs_default ? 1 : 0) != 0);
     std::vector<const FourStepKernel *> dit_vars;
     if (real_rows) {
         // only the variants with a real-input version
@@ -371,11 +393,15 @@ void C2CCore::run_stalled(const void *in, void *out, cudaStream_t st) const
 // ---------------------------------------------------------------------------
 // column FFTs
 
+// columns a tile of TILE_COL_SMALL
+static constexpr int SMALL_C = 4;
+
 void ColCore::init(int dtype_, int logl_, int variant_, bool allow_split, long long max_cols)
 {
     dtype = dtype_;
     logl = logl_;
     variant = variant_;
+    real2d = !allow_split;
     // Columns of up to 2^12 points run in one launch of tiles.  Longer ones
     // (the reference's FFTVert goes to 2^23 rows, fft_impl_generic.h:281-315)
     // run split; fp32 plain columns of 2^10 .. 2^12 also do on request
@@ -415,10 +441,18 @@ void ColCore::init(int dtype_, int logl_, int variant_, bool allow_split, long l
         split = true;
         return;
     }
+    // the full-width real 2D layout of long fp32 columns: plain columns, then
+    // the mirrored half by a fill pass (colsplit.cu)
+    if (variant == TILE_COL_HERM && dtype == GFFT_F32 && logl >= 9) {
+        herm_fill = true;
+        variant = TILE_COL_PLAIN;
+    }
     c = tile_widest(dtype, variant, logl, (int)env_ll("GFFT_COL_MAXC", 16));
     if (!c) fail(GFFT_ERR_UNSUPPORTED, "no column kernel for this length");
     k = tile_find(dtype, variant, logl, c);
     tw = tile_table(dtype, k, logl, c);
+    if (variant == TILE_COL_PLAIN && (ks = tile_find(dtype, TILE_COL_SMALL, logl, SMALL_C)))
+        tw_s = tile_table(dtype, ks, logl, SMALL_C);
 }
 
 void ColCore::release()
@@ -430,10 +464,27 @@ void ColCore::release()
 void ColCore::run(int inverse, const void *in, void *out, long long ncols, long long ld_in, long long ld_out,
                   long long batch, long long idist, long long odist, cudaStream_t st, double scale) const
 {
+    // The 4-column tiles of 16 points a thread:
+    // - few columns: while these tiles run in one wave of the 152 SMs they
+    //   finish sooner than the wide tiles of 64 points a thread (GB300, us a
+    //   call: 256 columns of 2^11 points 7.1 against 8.6, of 2^12 11.8 /
+    //   12.2; 1024 columns 13.5 / 11.6 and 24.0 / 23.6);
+    // - the column pass of real 2D transforms at 2^12, whatever its stride
+    //   (half- and full-width results hold the same bits), and 2^12 rows off
+    //   16-byte boundaries while the columns stay in L2 (96 of 129 MB):
+    //   boxes of 48 bytes for runs of 32 lose there what the copies gain
+    //   (real 4096 x 4096, forward and back, 166 us against 169 - 195).
+    //   Out of HBM the copies win: 4001 columns 88 us against 117.
     if (!split) {
-        check_cuda(launch_colpass(*k, inverse, (ncols + c - 1) / c, batch, in, out, ncols, ld_in, ld_out, idist,
-                                  odist, tw, nullptr, nullptr, 0, 0u, st, scale),
+        const bool odd = ((uintptr_t)in & 15u) != 0 || ld_in % 2 != 0;
+        const bool few = ks && (ncols * batch <= 152 * SMALL_C || (logl == 12 && (real2d || (odd && ((ncols * batch) << 15) <= (96LL << 20)))));
+        const int cw = few ? SMALL_C : c;
+        check_cuda(launch_colpass(few ? *ks : *k, inverse, (ncols + cw - 1) / cw, batch, in, out, ncols, ld_in, ld_out,
+                                  idist, odist, few ? tw_s : tw, nullptr, nullptr, 0, 0u, st, scale),
                    "launch column FFT");
+        if (herm_fill)
+            check_cuda(launch_herm_fill(dtype, out, 1LL << logl, 2 * (ncols - 1), ld_out, batch, odist, st),
+                       "launch Hermitian fill");
         return;
     }
     // rows in bit-reversed order: into natural order first (into out, or

@@ -66,6 +66,10 @@ struct ColCore {
     int dtype = 0, logl = 0, variant = 0, c = 0;
     const TileKernel *k = nullptr;
     const void *tw = nullptr;
+    // fp32 columns of 2^11 and 2^12 points: the short tile for few columns
+    const TileKernel *ks = nullptr;
+    const void *tw_s = nullptr;
+    bool real2d = false;  // the column pass of a real 2D transform
     // split column FFTs (columns longer than one tile, 2^13 .. 2^24 points,
     // and fp32 plain columns of 2^10 .. 2^12 on request): each column of
     // H = H1 * H2 points is two launches of short column FFTs per band of
@@ -87,7 +91,7 @@ struct ColCore {
     void release();
     long long launches(long long ncols, long long batch) const
     {
-        if (!split) return 1;
+        if (!split) return 1 + (herm_fill ? 1 : 0);
         return 2 * batch * ((ncols + band - 1) / band) + (rows_bitrev ? 1 : 0) + (herm_fill ? 1 : 0);
     }
     void run(int inverse, const void *in, void *out, long long ncols, long long ld_in, long long ld_out,

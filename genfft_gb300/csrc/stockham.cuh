@@ -64,7 +64,11 @@ struct StockhamPlan {
 //         (only touched when P > 1)
 //   tw  : the plan's twiddle table (StockhamPlan::TW elements)
 // SYNC() must synchronise every thread that shares the shared memory (the
-// whole CTA, or the group).
+// whole CTA, or the group).  READ_DONE() runs once this thread has read its
+// last exchange values: it touches the shared memory no more.  FIRST_WRITE()
+// runs before the thread's first write to it, with the first pass done in
+// registers (a caller whose threads still read their inputs there puts its
+// barrier in it).
 // twiddle loads through the read-only cache (tables in global memory)
 struct TwGlobal {
     template <typename T>
@@ -76,9 +80,15 @@ struct TwShared {
     __device__ __forceinline__ cpx<T> operator()(const cpx<T> *p) const { return *p; }
 };
 
-template <typename T, int LOGN, int E_, bool INV, typename TwLoad = TwGlobal, typename At, typename Sync>
+struct NoHook {
+    __device__ __forceinline__ void operator()() const {}
+};
+
+template <typename T, int LOGN, int E_, bool INV, typename TwLoad = TwGlobal, typename At, typename Sync,
+          typename ReadDone = NoHook, typename FirstWrite = NoHook>
 __device__ __forceinline__ void stockham_run(cpx<T> (&v)[StockhamPlan<T, LOGN, E_>::E], int t,
-                                             At at, const cpx<T> *__restrict__ tw, Sync SYNC)
+                                             At at, const cpx<T> *__restrict__ tw, Sync SYNC,
+                                             ReadDone READ_DONE = ReadDone{}, FirstWrite FIRST_WRITE = FirstWrite{})
 {
     using SP = StockhamPlan<T, LOGN, E_>;
     constexpr int E = SP::E, G = SP::G, P = SP::P, R0 = SP::R0;
@@ -90,13 +100,23 @@ __device__ __forceinline__ void stockham_run(cpx<T> (&v)[StockhamPlan<T, LOGN, E
 #pragma unroll
         for (int r = 0; r < R0; r++) u[r] = v[m + r * (E / R0)];
         dft<R0, INV, T>(u);
-        if constexpr (P == 1) {
+        if constexpr (P == 1 || !std::is_same_v<FirstWrite, NoHook>) {
 #pragma unroll
             for (int r = 0; r < R0; r++) v[m + r * (E / R0)] = u[r];
         } else {
             const int j = t + m * G;
 #pragma unroll
             for (int r = 0; r < R0; r++) at(j * R0 + r) = u[r];
+        }
+    }
+
+    if constexpr (P > 1 && !std::is_same_v<FirstWrite, NoHook>) {
+        FIRST_WRITE();
+#pragma unroll
+        for (int m = 0; m < E / R0; m++) {
+            const int j = t + m * G;
+#pragma unroll
+            for (int r = 0; r < R0; r++) at(j * R0 + r) = v[m + r * (E / R0)];
         }
     }
 
@@ -108,6 +128,7 @@ __device__ __forceinline__ void stockham_run(cpx<T> (&v)[StockhamPlan<T, LOGN, E
         SYNC();
 #pragma unroll
         for (int q = 0; q < E; q++) v[q] = at(t + q * G);
+        if constexpr (p == P - 1) READ_DONE();
         const int jm = t % Ns;  // Ns <= G, so j = t
         const cpx<T> *twp = tw + off + jm;
 #pragma unroll

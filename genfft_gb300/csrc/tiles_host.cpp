@@ -227,7 +227,7 @@ cudaError_t launch_colpass(const TileKernel &k, int inverse, long long tiles, lo
     // before it is written back
     const size_t eb = (size_t)k.elem_bytes;
     if (use_tma(k) && encode_fn() && aligned16(in) && (ld_in * eb) % 16 == 0 &&
-        (nbatch == 1 || (idist * eb) % 16 == 0) && ncols * (eb / 8) < (1LL << 32) && nbatch < (1LL << 31)) {
+        (nbatch == 1 || (idist * eb) % 16 == 0) && ncols * (eb / 8) < (1LL << 32) && nbatch < (1LL << 31) && tiles * nbatch < (1LL << 30)) {
         const int units = (int)(eb / 8);
         CUtensorMap map;
         const long long rows = k.tma_rows;
@@ -244,10 +244,42 @@ cudaError_t launch_colpass(const TileKernel &k, int inverse, long long tiles, lo
             if (e != cudaSuccess) return e;
             unsigned *err = device_error_word();
             const long long grid = persistent_grid(fn, k.tma_threads, k.tma_smem, tiles * nbatch);
+            // (the last one: k_colpass_tma's second tensor map, unused here)
             void *args[] = {(void *)&map, (void *)&out, (void *)&ncols, (void *)&ld_out, (void *)&odist,
                             (void *)&nbatch, (void *)&tw, (void *)&tw_lo, (void *)&tw_hi, (void *)&lo_bits,
-                            (void *)&nmask, (void *)&err, scale_p};
+                            (void *)&nmask, (void *)&err, scale_p, (void *)&map};
             return launch_pdl(fn, dim3((unsigned)grid), dim3(k.tma_threads), args, k.tma_smem, st);
+        }
+    }
+    // rows off 16-byte boundaries: even and odd rows through a tensor map
+    // each, twice the row stride apart and rounded down to a boundary (the
+    // bytes before an 8-byte aligned base are in its 16-byte granule).
+    // Batch strides have to keep every image's rows in step.
+    if (use_tma(k) && k.tmau_fwd && ((uintptr_t)in & 7u) == 0 && (nbatch == 1 || idist % 2 == 0) &&
+        ncols + 1 < (1LL << 31) && tiles * nbatch < (1LL << 30)) {
+        CUtensorMap map[2];
+        int skew = 0;
+        bool ok = true;
+        for (int r = 0; r < 2 && ok; r++) {
+            const uintptr_t base = (uintptr_t)in + (uintptr_t)(r * ld_in * (long long)eb);
+            const int off = (int)((base >> 3) & 1);
+            skew |= off << r;
+            ok = make_tensor_map_3d(&map[r], (const void *)(base & ~(uintptr_t)15), (unsigned long long)(ncols + off),
+                                    (unsigned long long)(k.tma_rows / 2), (unsigned long long)nbatch,
+                                    (unsigned long long)(2 * ld_in * eb),
+                                    (unsigned long long)((nbatch > 1 ? idist : k.tma_rows * ld_in) * eb),
+                                    (unsigned)(k.tma_c + 2), (unsigned)k.tmau_boxr);
+        }
+        if (ok) {
+            const void *fn = inverse ? k.tmau_inv : k.tmau_fwd;
+            cudaError_t e = ensure_smem(fn, k.tmau_smem);
+            if (e != cudaSuccess) return e;
+            unsigned *err = device_error_word();
+            const long long grid = persistent_grid(fn, k.tma_threads, k.tmau_smem, tiles * nbatch);
+            void *args[] = {(void *)&map[0], (void *)&out, (void *)&ncols, (void *)&ld_out, (void *)&odist,
+                            (void *)&nbatch, (void *)&tw, (void *)&tw_lo, (void *)&tw_hi, (void *)&skew,
+                            (void *)&nmask, (void *)&err, scale_p, (void *)&map[1]};
+            return launch_pdl(fn, dim3((unsigned)grid), dim3(k.tma_threads), args, k.tmau_smem, st);
         }
     }
     const void *fn = inverse ? k.inv : k.fwd;
@@ -276,7 +308,7 @@ cudaError_t launch_rowpass(const TileKernel &k, int inverse, long long tiles, lo
     void *scale_p = k.elem_bytes == 8 ? (void *)&scale_f : (void *)&scale;
     const size_t eb = (size_t)k.elem_bytes;
     if (use_tma(k) && aligned16(in) && (ld_in * eb) % 16 == 0 &&
-        (nbatch == 1 || (idist * eb) % 16 == 0)) {
+        (nbatch == 1 || (idist * eb) % 16 == 0) && tiles * nbatch < (1LL << 30)) {
         const void *fn = inverse ? k.tma_inv : k.tma_fwd;
         cudaError_t e = ensure_smem(fn, k.tma_smem);
         if (e != cudaSuccess) return e;

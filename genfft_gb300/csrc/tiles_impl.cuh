@@ -4,6 +4,7 @@
 
 #include "tiles.cuh"
 #include "tiles_tma.cuh"
+#include "tiles_pipe.cuh"
 #include "tiles_registry.h"
 #include "twiddle.h"
 #include "../../include/genfft_gb300.h"
@@ -85,7 +86,65 @@ struct TileReg {
         k.twcount = (size_t)SP::TW;
         k.fill = &tile_fill_tw<T, LOGL, E>;
         k.elem_bytes = (int)sizeof(cpx<T>);
+        k.e = SP::E;
+        k.g = SP::G;
         tile_register(sizeof(T) == 4 ? GFFT_F32 : GFFT_F64, V, LOGL, C, k);
+    }
+};
+
+// fp32 tiles of the pipelined kernels (tiles_pipe.cuh), NG groups and NB
+// stages, beside the plain kernels of the same arithmetic for inputs that
+// TMA copies cannot read
+template <int V, int LOGL, int C, int E, int NG, int NB, int NBU = NB>
+struct PipeReg {
+    PipeReg()
+    {
+        using T = float;
+        using SP = StockhamPlan<T, LOGL, E>;
+        TileKernel k;
+        if constexpr (V == TILE_ROW_PIPE) {
+            using Cfg = RowCfg<T, LOGL, C, E>;
+            using PCfg = PipeCfg<T, LOGL, C, E, NG, NB, LAND_ROW>;
+            k.fwd = (const void *)&k_rowpass<T, LOGL, C, E, false>;
+            k.inv = (const void *)&k_rowpass<T, LOGL, C, E, true>;
+            k.threads = Cfg::THREADS;
+            k.smem = Cfg::SMEM;
+            k.tma_fwd = (const void *)&pipe::k_rowpass_tma<T, LOGL, C, E, NG, NB, false>;
+            k.tma_inv = (const void *)&pipe::k_rowpass_tma<T, LOGL, C, E, NG, NB, true>;
+            k.tma_threads = PCfg::THREADS;
+            k.tma_smem = PCfg::SMEM;
+            k.tma_row = true;
+        } else {
+            using Cfg = ColCfg<T, LOGL, C, E>;
+            using PCfg = PipeCfg<T, LOGL, C, E, NG, NB, LAND_COL>;
+            constexpr int twm = V == TILE_COL_TWP ? 3 : V == TILE_COL_TWB ? 4 : 0;
+            k.fwd = (const void *)&k_colpass<T, LOGL, C, E, false, twm, false>;
+            k.inv = (const void *)&k_colpass<T, LOGL, C, E, true, twm, false>;
+            k.threads = Cfg::THREADS;
+            k.smem = Cfg::SMEM;
+            k.tma_fwd = (const void *)&pipe::k_colpass_tma<T, LOGL, C, E, NG, NB, false, twm>;
+            k.tma_inv = (const void *)&pipe::k_colpass_tma<T, LOGL, C, E, NG, NB, true, twm>;
+            k.tma_threads = PCfg::THREADS;
+            k.tma_smem = PCfg::SMEM;
+            k.tma_boxr = PCfg::BOXR;
+            k.tma_rows = PCfg::N;
+            k.tma_c = C;
+            k.t12 = twm != 0;
+            if constexpr (V == TILE_COL_PLAIN) {
+                using UCfg = PipeCfg<T, LOGL, C, E, NG, NBU, LAND_COLU>;
+                k.tmau_fwd = (const void *)&pipe::k_colpass_tma<T, LOGL, C, E, NG, NBU, false, 0, true>;
+                k.tmau_inv = (const void *)&pipe::k_colpass_tma<T, LOGL, C, E, NG, NBU, true, 0, true>;
+                k.tmau_smem = UCfg::SMEM;
+                k.tmau_boxr = UCfg::BOXR;
+            }
+        }
+        k.tma_stages = 3;
+        k.twcount = (size_t)SP::TW;
+        k.fill = &tile_fill_tw<T, LOGL, E>;
+        k.elem_bytes = (int)sizeof(cpx<T>);
+        k.e = SP::E;
+        k.g = SP::G;
+        tile_register(GFFT_F32, V, LOGL, C, k);
     }
 };
 

@@ -16,7 +16,10 @@ enum TileVariant {
     TILE_COL_BITREV = 2,  // column FFT, bit-reversed row order on input
     TILE_ROW_XPOSE = 3,   // row pass with transposed store
     TILE_COL_HERM = 4,    // column FFT + Hermitian mirror store (real 2D)
-    TILE_COL_TWB = 5      // column pass with the W_N^(batch * row) twiddle (split column FFTs)
+    TILE_COL_TWB = 5,     // column pass with the W_N^(batch * row) twiddle (split column FFTs)
+    TILE_COL_TWP = 6,     // TILE_COL_TW4 with 32 or 64 points a thread (tiles_pipe.cuh)
+    TILE_COL_SMALL = 8,   // TILE_COL_PLAIN for few columns (one wave of short tiles)
+    TILE_ROW_PIPE = 7     // TILE_ROW_XPOSE with 32 or 64 points a thread (tiles_pipe.cuh)
 };
 
 struct TileKernel {
@@ -34,7 +37,14 @@ struct TileKernel {
     int tma_boxr = 0;  // column pass: rows per tensor box
     int tma_rows = 0;  // column pass: column length (tensor rows)
     int tma_c = 0;     // columns per tile
-    int tma_stages = 0;  // 2 double-buffered, 1 single buffer
+    int tma_stages = 0;  // 2 double-buffered, 1 single buffer, 3 the tiles_pipe.cuh kernels
+    // TILE_COL_PLAIN of tiles_pipe.cuh: the version for rows off 16-byte
+    // boundaries (tma_boxr rows of each parity a box, tma_c + 2 columns)
+    const void *tmau_fwd = nullptr, *tmau_inv = nullptr;
+    size_t tmau_smem = 0;
+    int tmau_boxr = 0;
+    int e = 0, g = 0;    // points a thread, threads a column (row)
+    bool t12 = false;    // twiddle tables t1 / t2 (tiles_pipe.cuh), not the lo / hi split
     bool tma_row = false;  // a row-pass kernel (for the GFFT_TMA1 knob)
 };
 
