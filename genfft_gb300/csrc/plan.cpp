@@ -63,21 +63,22 @@ static void wn_tables(int dtype, int logn, int *lo_bits, const void **lo, const 
     *hi = cached_table(key + "/hi", dtype, N >> *lo_bits, fill(N >> *lo_bits, 1LL << *lo_bits));
 }
 
-// the inter-pass twiddle tables of a tiles_pipe.cuh kernel over N = 2^logn:
-// t1[e] = W_N^e for e < N / E, t2[e] = W_N^(G e) for e < N / G
+// the inter-pass twiddle tables of a tiles_pipe.cuh kernel over N = 2^logn,
+// E points a thread, G threads a column:
+// t1[f][t] = W_N^(f t), t < G, and t2[f][q] = W_N^(G f q), q < E, for f < N / (E G)
 static void t12_tables(int dtype, int logn, const TileKernel *k, const void **t1, const void **t2)
 {
-    const long long N = 1LL << logn;
-    auto fill = [N](long long count, long long mul) {
-        return [N, count, mul](void *buf) {
-            for (long long e = 0; e < count; e++)
-                forward_root<float>(e * mul, N, &((float *)buf)[2 * e], &((float *)buf)[2 * e + 1]);
+    const long long N = 1LL << logn, e = k->e, g = k->g, F = N / (e * g);
+    auto fill = [N, F](long long width, long long mul) {
+        return [N, F, width, mul](void *buf) {
+            float *o = static_cast<float *>(buf);
+            for (long long f = 0; f < F; f++)
+                for (long long j = 0; j < width; j++, o += 2) forward_root<float>(f * j * mul, N, o, o + 1);
         };
     };
-    const std::string key = "t12/" + std::to_string(logn) + "/";
-    const long long n1 = N / k->e, n2 = N / k->g;
-    *t1 = cached_table(key + "1/" + std::to_string(k->e), dtype, n1, fill(n1, 1));
-    *t2 = cached_table(key + "2/" + std::to_string(k->g), dtype, n2, fill(n2, k->g));
+    const std::string key = "t12/" + std::to_string(logn) + "/" + std::to_string(e) + "/" + std::to_string(g);
+    *t1 = cached_table(key + "/1", dtype, F * g, fill(g, 1));
+    *t2 = cached_table(key + "/2", dtype, F * e, fill(e, g));
 }
 
 static const void *tile_table(int dtype, const TileKernel *k, int logl, int c)
@@ -90,7 +91,7 @@ static const void *tile_table(int dtype, const TileKernel *k, int logl, int c)
 // ---------------------------------------------------------------------------
 // C2C
 
-void C2CCore::init(int dtype_, int logn_, long long batch_hint, int path, bool real_rows)
+void C2CCore::init(int dtype_, int logn_, long long batch_hint, int path, bool real_rows, int log_a)
 {
     dtype = dtype_;
     logn = logn_;
@@ -103,7 +104,7 @@ void C2CCore::init(int dtype_, int logn_, long long batch_hint, int path, bool r
     }
     if (logn > 24) fail(GFFT_ERR_INVALID_SIZE, "transform length above 2^24 is not supported");
     // N = A * B, A = column-FFT length, B = row-FFT length, both <= 2^12
-    logA = logn / 2;
+    logA = log_a ? log_a : logn / 2;
     logB = logn - logA;
     const long long N = 1LL << logn;
     const int d = dtype;
@@ -120,10 +121,16 @@ void C2CCore::init(int dtype_, int logn_, long long batch_hint, int path, bool r
     // (GFFT_PIPE=1 / 0 overrides).  GFFT_FS, GFFT_FS_PAIR and GFFT_3PASS
     // still name the paths they did.
     const long long want_pipe = env_ll("GFFT_PIPE", -1);
+    // (2^17 with 512-point columns: 2^17 x 333 225 us against 246 the other way)
+    const int la = log_a ? log_a : std::max(logn / 2, std::min(9, logn - 8));
     const bool pipe = dtype == GFFT_F32 && path <= 0 && !real_rows && logn >= 16 &&
-                      (want_pipe > 0 || (want_pipe < 0 && logn >= 17 && env_ll("GFFT_3PASS", 0) <= 0 &&
+                      (log_a > 0 || want_pipe > 0 || (want_pipe < 0 && logn >= 17 && env_ll("GFFT_3PASS", 0) <= 0 &&
                                          env_ll("GFFT_FS", 0) == 0 && env_ll("GFFT_FS_PAIR", 0) == 0)) &&
-                      tile_widest(dtype, TILE_COL_TWP, logA, maxc) && tile_widest(dtype, TILE_ROW_PIPE, logB, maxc);
+                      tile_widest(dtype, TILE_COL_TWP, la, maxc) && tile_widest(dtype, TILE_ROW_PIPE, logn - la, maxc);
+    if (pipe) {
+        logA = la;
+        logB = logn - la;
+    }
     const int vcol = pipe ? TILE_COL_TWP : TILE_COL_TW4, vrow = pipe ? TILE_ROW_PIPE : TILE_ROW_XPOSE;
     ccol = tile_widest(dtype, vcol, logA, maxc);
     crow = tile_widest(dtype, vrow, logB, maxc);
@@ -301,12 +308,20 @@ void C2CCore::run(int inverse, const void *in, void *out, long long batch, long 
         const long long nb = std::min(group, batch - g0);
         const char *src = static_cast<const char *>(in) + (size_t)(g0 * idist) * eb;
         char *dst = static_cast<char *>(out) + (size_t)(g0 * odist) * eb;
+        // Out of HBM the 512-point columns ask for more than it can give:
+        // with the next copy started after a tile's stores (see launch_colpass)
+        // fewer are queued and the whole is faster; out of L2 the copies have
+        // to run ahead.  GB300, us, early / late: 2^18 x 512 717 / 674,
+        // 2^19 x 128 377 / 355, 2^17 x 512 375 / 340; 2^18 x 64 (134 MB)
+        // 99 / 107.  With 1024-point columns there is nothing to gain
+        // (2^20 x 128 733 / 737).
+        const bool late = logA <= 9 && N * nb * (long long)eb > (200LL << 20);
         // column pass: B columns of A points (row stride B) into the workspace
         check_cuda(launch_colpass(*kcol, inverse, B / ccol, nb, src, ws, B, B, B, idist, N, tw_col, tw_lo, tw_hi,
-                                  lo_bits, nmask, st),
+                                  lo_bits, nmask, st, 1.0, late),
                    "launch column pass");
         // row pass: A rows of B points, stored transposed (stride A)
-        check_cuda(launch_rowpass(*krow, inverse, A / crow, nb, ws, dst, A, B, A, N, odist, tw_row, st, scale),
+        check_cuda(launch_rowpass(*krow, inverse, A / crow, nb, ws, dst, A, B, A, N, odist, tw_row, st, scale, late),
                    "launch row pass");
     }
 }
@@ -546,6 +561,16 @@ void R2CCore::init(int dtype_, int logn_, int half_, long long batch_hint)
                           [d, lh](void *buf) { r2c_twiddle_fill(d, lh, buf); });
         return;
     }
+    // pipelined passes (real_pipe.cu): rows of 2^9, columns of 2^8 .. 2^12
+    // (GB300, us, n = 2^20 x 64: 234 against 314)
+    const int lr = realpipe_logl();
+    if (dtype == GFFT_F32 && half == 1 && lh >= 8 + lr && lh <= 12 + lr && env_ll("GFFT_R2C_FUSED_DIT", 1) != 0 &&
+        env_ll("GFFT_R2C_FS", 0) == 0 && env_ll("GFFT_PIPE", 1) != 0) {
+        c2c.init(dtype, lh, batch_hint, 0, false, lh - lr);
+        tw_rowdit = cached_table("realpipe", d, realpipe_twiddle_count(), [](void *buf) { realpipe_twiddle_fill(buf); });
+        algo = 5;
+        return;
+    }
     // the DIT fused into the row pass of a four-step split of n/2 (fp32)
     const RowDitKernel *k = rowdit_find(dtype, lh - lh / 2);
     if (k && env_ll("GFFT_R2C_FUSED_DIT", 1) != 0) {
@@ -580,7 +605,7 @@ void R2CCore::init(int dtype_, int logn_, int half_, long long batch_hint)
 int R2CCore::launches(long long batch) const
 {
     if (algo == 2) return c2c.launches(batch) + 1;
-    if (algo == 3 || algo == 4) return c2c.launches(batch);
+    if (algo >= 3) return c2c.launches(batch);
     return 1;
 }
 
@@ -596,7 +621,7 @@ void R2CCore::run(const void *in, void *out, long long batch, long long idist, l
     } else if (algo == 4 && mode == 0 && c2c.run_persistent(0, in, out, batch, idist / 2, odist, st, scale, dtw)) {
         // one persistent launch: column items, then row items that apply
         // the DIT adjustment and store the half spectrum
-    } else if ((algo == 3 || algo == 4) && mode == 0) {
+    } else if (algo >= 3 && mode == 0) {
         // column pass of the n/2-point split into the workspace, then the
         // row pass with the DIT adjustment fused, straight into the spectrum
         // (also the persistent plan's path for inputs its tensor copies
@@ -610,7 +635,10 @@ void R2CCore::run(const void *in, void *out, long long batch, long long idist, l
             check_cuda(launch_colpass(*c2c.kcol, 0, B / c2c.ccol, nb, src, c2c.ws, B, B, B, idist / 2, N, c2c.tw_col,
                                       c2c.tw_lo, c2c.tw_hi, c2c.lo_bits, (unsigned)(N - 1), st),
                        "launch column pass");
-            check_cuda(launch_rowpass_dit(*rowdit, c2c.ws, dst, A, nb, N, odist, tw_rowdit, dtw, st, scale),
+            if (algo == 5)
+                check_cuda(launch_rowdit_pipe(c2c.ws, dst, A, nb, N, odist, tw_rowdit, dtw, st, scale),
+                           "launch row pass with DIT");
+            else check_cuda(launch_rowpass_dit(*rowdit, c2c.ws, dst, A, nb, N, odist, tw_rowdit, dtw, st, scale),
                        "launch row pass with DIT");
         }
     } else {
@@ -648,6 +676,13 @@ void C2RCore::init(int dtype_, int logn_, long long batch_hint)
         }
         return;
     }
+    // pipelined passes (real_pipe.cu): columns of 2^9, rows of 2^8 .. 2^12
+    const int lr = realpipe_logl();
+    if (dtype == GFFT_F32 && lh >= 8 + lr && lh <= 12 + lr && env_ll("GFFT_PIPE", 1) != 0) {
+        c2c.init(dtype, lh, batch_hint, 0, false, lr);
+        algo = 3;
+        return;
+    }
     algo = 2;
     c2c.init(dtype, lh, batch_hint);
 }
@@ -655,6 +690,7 @@ void C2RCore::init(int dtype_, int logn_, long long batch_hint)
 int C2RCore::launches(long long batch) const
 {
     if (algo == 2) return c2c.launches(batch) + 1;
+    if (algo == 3) return c2c.launches(batch);
     return 1;
 }
 
@@ -666,6 +702,20 @@ void C2RCore::run(const void *in, void *out, long long batch, long long idist, l
     } else if (algo == 1 && !(fold_split && wmode == 2)) {
         check_cuda(launch_c2r_fused(dtype, logn - 1, wmode, in, out, batch, idist, odist, tw, dtw, st, scale),
                    "launch fused C2R");
+    } else if (algo == 3 && wmode != 2) {
+        const long long A = 1LL << c2c.logA, B = 1LL << c2c.logB, N = A * B;
+        const size_t eb = cplx_bytes(dtype);
+        for (long long g0 = 0; g0 < batch; g0 += c2c.group) {
+            const long long nb = std::min(c2c.group, batch - g0);
+            const char *src = static_cast<const char *>(in) + (size_t)(g0 * idist) * eb;
+            char *dst = static_cast<char *>(out) + (size_t)(g0 * (odist / 2)) * eb;
+            check_cuda(launch_c2rcol_pipe(src, c2c.ws, B, nb, idist, c2c.tw_col, c2c.tw_lo, c2c.tw_hi, dtw, wmode == 1,
+                                          st),
+                       "launch C2R column pass");
+            check_cuda(launch_rowpass(*c2c.krow, 1, A / c2c.crow, nb, c2c.ws, dst, A, B, A, N, odist / 2, c2c.tw_row, st,
+                                      scale),
+                       "launch row pass");
+        }
     } else {
         const long long H = 1LL << (logn - 1);
         // Z' (n/2 complex = the n output reals) into the output buffer, then

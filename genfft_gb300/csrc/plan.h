@@ -45,7 +45,8 @@ struct C2CCore {
     // path: -1 the measured default (or GFFT_FS), 1 the persistent
     // four-step kernel, 0 the tile launches.  real_rows (with path 1): a
     // variant with a real-input version, scheduled for its row items
-    void init(int dtype, int logn, long long batch_hint, int path = -1, bool real_rows = false);
+    // log_a: log2 of the column length A (0: half of logn)
+    void init(int dtype, int logn, long long batch_hint, int path = -1, bool real_rows = false, int log_a = 0);
     void release();
     int launches(long long batch) const;
     // strides in complex elements; four-step needs unit element strides
@@ -137,7 +138,10 @@ struct R2CCore {
 // extension (imaginary parts of the DC and Nyquist bins ignored)
 struct C2RCore {
     int dtype = 0, logn = 0;
-    int algo = 0;  // 0 n == 1, 1 fused, 2 pre-pass + C2C(n/2) inverse
+    // 0 n == 1, 1 fused, 2 pre-pass + C2C(n/2) inverse, 3 pipelined column
+    // pass that forms Z' + row pass (real_pipe.cu; the folded full spectrum
+    // as 2)
+    int algo = 0;
     const void *tw = nullptr, *dtw = nullptr;
     // algo 1 whose folded full-spectrum input (2 n/2 bins) does not fit the
     // fused kernel's shared memory: that mode takes the algo 2 route
@@ -166,6 +170,19 @@ struct TCCore {
     void run(int inverse, const void *in, void *out, long long batch, long long idist, long long odist,
              long long istride, long long ostride, cudaStream_t st, double scale = 1.0) const;
 };
+
+// ---- pipelined real transforms, fp32 n = 2^18 .. 2^22 (real_pipe.cu) -----
+int realpipe_logl();  // log2 of the row (R2C) / column (C2R) length
+size_t realpipe_twiddle_count();
+void realpipe_twiddle_fill(void *buf);
+// row pass with the DIT over `A` rows a transform, workspace to half spectrum
+cudaError_t launch_rowdit_pipe(const void *in, void *out, long long A, long long batch, long long idist,
+                               long long odist, const void *tw, const void *dtw, cudaStream_t st, double scale);
+// half spectrum to the workspace: Z' and the column pass of the inverse over
+// B columns (t1, t2: the inter-pass twiddles); half_interior: interior bins
+// halved (adjoint of the half-spectrum R2C)
+cudaError_t launch_c2rcol_pipe(const void *in, void *ws, long long B, long long batch, long long idist, const void *tw,
+                               const void *t1, const void *t2, const void *dtw, bool half_interior, cudaStream_t st);
 
 // ---- kernels in real.cu --------------------------------------------------
 int r2c_fused_max_logh(int dtype);

@@ -7,7 +7,7 @@ namespace gfft {
 // (length, columns or rows a tile, points a thread, groups, stages)
 #define P(V, L, C, E, NG, NB) static PipeReg<V, L, C, E, NG, NB> pipe_##V##_##L##_##C;
 #define P2(L, C, E, NG, NB) P(TILE_COL_TWP, L, C, E, NG, NB) P(TILE_ROW_PIPE, L, C, E, NG, NB)
-P2(8, 16, 32, 4, 6) P2(9, 16, 32, 2, 3) P2(10, 8, 32, 2, 3) P2(11, 8, 64, 1, 1) P2(12, 4, 64, 1, 1)
+P2(8, 16, 32, 4, 4) P2(9, 16, 32, 2, 2) P2(10, 8, 32, 2, 2) P2(11, 8, 64, 1, 1) P2(12, 4, 64, 1, 1)
 #undef P2
 #undef P
 }  // namespace gfft

@@ -3,10 +3,9 @@
 #include "tiles_impl.cuh"
 
 namespace gfft {
-#define P(V, L, C, E, NG, NB, NBU) static PipeReg<V, L, C, E, NG, NB, NBU> pipe_##V##_##L##_##C;
-// (NBU: stages of the version for rows off 16-byte boundaries)
-#define P2(L, C, E, NG, NB, NBU) P(TILE_COL_PLAIN, L, C, E, NG, NB, NBU)
+// (length, columns a tile, points a thread, groups, stages, stages of the
+// version for rows off 16-byte boundaries)
+#define P2(L, C, E, NG, NB, NBU) static PipeReg<TILE_COL_PLAIN, L, C, E, NG, NB, NBU> pipe_plain_##L##_##C;
 P2(9, 16, 32, 2, 3, 3) P2(10, 8, 32, 2, 3, 2) P2(11, 8, 64, 1, 1, 1) P2(12, 4, 64, 1, 1, 1)
 #undef P2
-#undef P
 }  // namespace gfft

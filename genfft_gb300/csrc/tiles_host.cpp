@@ -26,6 +26,8 @@ std::mutex &reg_mu()
     return m;
 }
 
+}  // namespace
+
 int sm_count()
 {
     static std::mutex mu;
@@ -40,8 +42,6 @@ int sm_count()
     cache[dev] = n;
     return n;
 }
-
-}  // namespace
 
 cudaError_t ensure_smem(const void *fn, size_t smem)
 {
@@ -217,8 +217,9 @@ int tile_widest(int dtype, int variant, int logl, int max_c)
 cudaError_t launch_colpass(const TileKernel &k, int inverse, long long tiles, long long nbatch,
                            const void *in, void *out, long long ncols, long long ld_in, long long ld_out,
                            long long idist, long long odist, const void *tw, const void *tw_lo,
-                           const void *tw_hi, int lo_bits, unsigned nmask, cudaStream_t st, double scale)
+                           const void *tw_hi, int lo_bits, unsigned nmask, cudaStream_t st, double scale, bool late)
 {
+    if (k.tma_stages == 3) nmask = late;  // (the pipelined kernels' parameter in its place)
     // the kernels take the scale as their element type
     float scale_f = (float)scale;
     void *scale_p = k.elem_bytes == 8 ? (void *)&scale_f : (void *)&scale;
@@ -302,7 +303,7 @@ cudaError_t launch_colpass(const TileKernel &k, int inverse, long long tiles, lo
 
 cudaError_t launch_rowpass(const TileKernel &k, int inverse, long long tiles, long long nbatch,
                            const void *in, void *out, long long nrows, long long ld_in, long long ostride,
-                           long long idist, long long odist, const void *tw, cudaStream_t st, double scale)
+                           long long idist, long long odist, const void *tw, cudaStream_t st, double scale, bool late)
 {
     float scale_f = (float)scale;
     void *scale_p = k.elem_bytes == 8 ? (void *)&scale_f : (void *)&scale;
@@ -314,8 +315,10 @@ cudaError_t launch_rowpass(const TileKernel &k, int inverse, long long tiles, lo
         if (e != cudaSuccess) return e;
         unsigned *err = device_error_word();
         const long long grid = persistent_grid(fn, k.tma_threads, k.tma_smem, tiles * nbatch);
+        unsigned late_u = late;
         void *args[] = {(void *)&in,    (void *)&out,   (void *)&nrows, (void *)&ld_in, (void *)&ostride,
-                        (void *)&idist, (void *)&odist, (void *)&nbatch, (void *)&tw, (void *)&err, scale_p};
+                        (void *)&idist, (void *)&odist, (void *)&nbatch, (void *)&tw, (void *)&err, scale_p,
+                        (void *)&late_u};
         return launch_pdl(fn, dim3((unsigned)grid), dim3(k.tma_threads), args, k.tma_smem, st);
     }
     const void *fn = inverse ? k.inv : k.fwd;

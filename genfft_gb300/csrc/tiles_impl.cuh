@@ -93,7 +93,7 @@ struct TileReg {
 };
 
 // fp32 tiles of the pipelined kernels (tiles_pipe.cuh), NG groups and NB
-// stages, beside the plain kernels of the same arithmetic for inputs that
+// stages (NBU: of the version for rows off 16-byte boundaries), beside the plain kernels of the same arithmetic for inputs that
 // TMA copies cannot read
 template <int V, int LOGL, int C, int E, int NG, int NB, int NBU = NB>
 struct PipeReg {

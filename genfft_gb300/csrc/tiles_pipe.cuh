@@ -2,19 +2,22 @@
 // 2^9 .. 2^12 points with 32 or 64 points a thread: two Stockham passes and
 // one shared-memory exchange where 16 points a thread need three and two.
 //
-// A CTA (one per SM) holds NG thread groups and NB shared-memory stages.
-// Each group works on a tile of C columns (rows) by itself, on its own named
+// A CTA (one per SM) holds NG thread groups and NB >= NG shared-memory stages.
+// A group works on a tile of C columns (rows) by itself, on its own named
 // barriers; tile i of the CTA goes to group i mod NG and stage i mod NB.  A
 // tile's TMA copy lands in its stage, the exchange runs in place there, and
-// as soon as the group has read its last exchange values one thread starts
-// the copy of tile i + NB into the stage.  So one group's butterflies and
-// stores overlap the other's and the copies in flight, and a barrier never
-// stops the whole SM.
+// once the group has read its last exchange values one thread starts the copy
+// of tile i + NB into the stage.  So one group's butterflies and stores
+// overlap the others' and the copies in flight, and a barrier never stops the
+// whole SM.  The four-step passes take a stage a group, the column FFTs of the
+// 2D and column transforms, whose data is in L2 more often, one more (GB300,
+// us, with / without it: 2^10 columns 5000 16.6 / 19.8; C2C 2^20 x 128
+// 794 / 733, 2^19 x 128 389 / 355: more copies in flight than HBM serves well).
 //
 // What bounds them (GB300; 6683 GB/s is the copy rate; GB/s of one pass over
-// a 1 GB batch in a kernel probe, every group and stage count that fits tried):
-//   columns  512 x 16 (2 groups of 256, 3 stages)  6094   HBM
-//           1024 x  8 (2 groups of 256, 3 stages)  5563   HBM, 64-byte runs
+// a 1 GB batch in a kernel probe):
+//   columns  512 x 16 (2 groups of 256)            6094   HBM
+//           1024 x  8 (2 groups of 256)            5563   HBM, 64-byte runs
 //           2048 x  8 (1 group of 256, 64 points)  5674   issue, 8 warps
 //           4096 x  4 (1 group of 256, 64 points)  4655   32-byte runs
 //   rows     512 x 16  6312, 1024 x 8  6139, 2048 x 8  5998
@@ -28,15 +31,17 @@
 // C2C through two such passes, GB300, GB/s forward, against the paths before
 // (persistent four-step 2^17 .. 2^19, 16-point tiles 2^20, three passes of
 // short tiles 2^21 .. 2^24), 1 GB batches:
-//   2^17 2968 / 2385   2^18 3075 / 2103   2^19 2732 / 1951   2^20 2697 / 2110
-//   2^21 2850 / 2098   2^22 2889 / 2071   2^23 2788 / 2003   2^24 2651 / 1916
+//   2^17 3157 / 2385   2^18 3189 / 2103   2^19 3024 / 1951   2^20 2931 / 2110
+//   2^21 2925 / 2098   2^22 2851 / 2071   2^23 2788 / 2003   2^24 2651 / 1916
 // and one transform: 2^17 8.9 us / 16.2, 2^20 11.4 / 20.6, 2^24 115 / 146.
 //
 // Inter-pass twiddle W_N^(f k), k = t + q G, f the column (TWM 3) or the
 // batch index (TWM 4): W_N^(f t) * W_N^(G f q) from two tables of directly
-// rounded roots, t1[f t] (N / E entries) and t2[f q] (N / G entries).  A
-// thread loads one t1 value a tile and the group stages the E x C t2 values
-// it needs, where the hi / lo split costs two scattered loads a point.
+// rounded roots, t1[f][t] (G a row) and t2[f][q] (E a row).  A thread loads
+// one t1 value a tile and the group stages the E x C t2 values it needs,
+// where the hi / lo split costs two scattered loads a point.  (Indexed by the
+// products f t and f q the tables are as small, but every load is a sector of
+// its own: a third of the column pass's L2 reads.)
 #pragma once
 
 #include "tiles_tma.cuh"
@@ -95,19 +100,19 @@ struct PipeCfg {
     static constexpr int BW = LD == LAND_COLU ? C + 2 : C;
     static constexpr int LAND = LD == LAND_ROW ? RP * C : N * BW;
     static constexpr int STAGE = StageRound<T, cmax<PITCH * C, LAND>::value>::value;
-    static constexpr int T2 = LD == LAND_COL ? C * SP::E : 0;  // staged t2 values of a group's tile
+    static constexpr int T2 = LD == LAND_COL ? C * SP::E : 0;  // staged t2 values of a group's tile (two buffers)
     // rows per tensor box (LAND_COLU: of the even or the odd rows)
     static constexpr int BOXR = N < 256 ? N : 256;
-    static constexpr size_t BAR_OFF = ((size_t)NB * STAGE + SP::TW + NG * T2) * sizeof(cpx<T>);
+    static constexpr size_t BAR_OFF = ((size_t)NB * STAGE + (size_t)NG * 2 * T2 + SP::TW) * sizeof(cpx<T>);
     static constexpr size_t SMEM = BAR_OFF + 128;  // + barriers and sequence numbers
     static_assert(SMEM <= 227 * 1024, "stages and tables must fit one CTA");
-    static_assert(GT % 32 == 0 && 1 + 2 * NG <= 16 && NB * 12 <= 128, "whole warps, barrier ids, barrier words");
+    static_assert(GT % 32 == 0 && 1 + 2 * NG <= 16 && NB >= NG && NB * 12 <= 128, "whole warps, barrier ids, barrier words");
 };
 
 // Stage hand-over.  An mbarrier's parity names two phases, so a group may
-// wait for tile i only once the copy of tile i has been armed: a stage goes
-// from group to group, and a group that got there while the copy of tile
-// i - NB was still in flight would take that phase's parity for its own.
+// wait for tile i only once the copy of tile i has been armed: with NB > NG a
+// stage goes from group to group, and a group that got there while the copy of
+// tile i - NB was still in flight would take that phase's parity for its own.
 // Whoever arms tile i's copy publishes i in seq[i mod NB] first thing after.
 __device__ __forceinline__ void seq_publish(int *seq, int i)
 {
@@ -119,7 +124,8 @@ __device__ __forceinline__ int seq_read(const int *seq)
     asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];" : "=r"(v) : "r"(smem_u32(seq)) : "memory");
     return v;
 }
-// wait (bounded) until tile i's copy is armed and has landed
+// wait (bounded) until tile i's copy is armed and has landed; the warp leaves
+// it converged
 __device__ __forceinline__ bool stage_wait(uint64_t *full, const int *seq, int i, uint32_t parity)
 {
     bool ok = true;
@@ -132,9 +138,10 @@ __device__ __forceinline__ bool stage_wait(uint64_t *full, const int *seq, int i
     return ok;
 }
 
-// The loop both passes share.  issue(i) starts the copy of the CTA's tile i
-// (thread 0 of a group), body(i, stage, ok) transforms and stores tile i and
-// returns false when its copy did not land in time.
+// The loop the passes share: tile i of the CTA is tile w0 + i step of the
+// launch.  issue(i) starts its copy (one thread; nothing past the last tile),
+// body(i, stage, parity) transforms and stores it, starts the copy of tile
+// i + NB and returns false when its own did not land in time.
 template <typename Cfg, typename Issue, typename Body>
 __device__ __forceinline__ void pipe_loop(uint64_t *full, const int *seq, unsigned *err, int w0, int step, int total,
                                           Issue issue, Body body)
@@ -156,6 +163,33 @@ __device__ __forceinline__ void pipe_loop(uint64_t *full, const int *seq, unsign
     }
 }
 
+// 8-byte asynchronous copy global -> shared, and the wait for this thread's
+__device__ __forceinline__ void cp_async8(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Frees a stage once the whole group has read it and starts the next copy
+// into it.  Every warp calls stage_read after its last read; the issuing warp
+// calls stage_refill, the only one to wait for the others, right after it or
+// (`late`, see C2CCore::run) once its own stores are out.
+__device__ __forceinline__ void stage_read(int bar, int nthreads, int tid)
+{
+    if (tid >= 32) bar_group_arrive(bar, nthreads);
+}
+template <typename Issue>
+__device__ __forceinline__ void stage_refill(int bar, int nthreads, int tid, bool landed, int next, Issue issue)
+{
+    if (tid >= 32) return;
+    bar_group(bar, nthreads);
+    if (tid == 0 && landed) {
+        fence_proxy_async_smem();
+        issue(next);
+    }
+    __syncwarp();
+}
+
 namespace pipe {
 
 // Column pass: see k_colpass (tiles.cuh); the tensor map views the input as
@@ -173,7 +207,7 @@ template <typename T, int LOGL, int C, int E_, int NG, int NB, bool INV, int TWM
 __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU : LAND_COL>::THREADS, 1)
     k_colpass_tma(const __grid_constant__ CUtensorMap map, cpx<T> *__restrict__ out, long long ncols, long long ld_out,
               long long odist, long long nbatch, const cpx<T> *__restrict__ tw, const cpx<T> *__restrict__ t1,
-              const cpx<T> *__restrict__ t2, int skew, unsigned, unsigned *err, T scale,
+              const cpx<T> *__restrict__ t2, int skew, unsigned late, unsigned *err, T scale,
               const __grid_constant__ CUtensorMap map1)
 {
     using Cfg = PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU : LAND_COL>;
@@ -187,9 +221,8 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU 
     cpx<T> *const tws = stage0 + (size_t)NB * Cfg::STAGE;
     uint64_t *const full = reinterpret_cast<uint64_t *>(smem_raw + Cfg::BAR_OFF);
     int *const seq = reinterpret_cast<int *>(full + NB);
-
     const int grp = threadIdx.x / GT, tid = threadIdx.x - grp * GT;
-    cpx<T> *const t2s = tws + SP::TW + grp * Cfg::T2;
+    cpx<T> *const t2b = tws + SP::TW + grp * 2 * Cfg::T2;
     const int bar = 1 + 2 * grp;
     const int s = tid % C, t = tid / C;
     // (tiles of 4096 points and more: their count fits 31 bits, and 32-bit
@@ -211,8 +244,8 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU 
         const int w = w0 + i * step;
         if (w >= total) return;
         const int buf = i % NB;
-        const int b = (int)((unsigned)w / (unsigned)tiles), c0 = (w - b * tiles) * C;
         cpx<T> *const S = stage0 + (size_t)buf * Cfg::STAGE;
+        const int b = (int)((unsigned)w / (unsigned)tiles), c0 = (w - b * tiles) * C;
         // out-of-range columns of the last tile are zero-filled and still counted
         mbar_arrive_expect_tx(&full[buf], (uint32_t)(N * Cfg::BW * sizeof(cpx<T>)));
         seq_publish(&seq[buf], i);
@@ -227,19 +260,22 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU 
     };
     pipe_loop<Cfg>(full, seq, err, w0, step, total, issue, [&](int i, int buf, uint32_t par) {
         const int w = w0 + i * step;
+        cpx<T> *const S = stage0 + (size_t)buf * Cfg::STAGE;
         const int wb = (int)((unsigned)w / (unsigned)tiles);
         const long long b = wb, col = (long long)(w - wb * tiles) * C + s;
         const bool active = col < ncols;
-        cpx<T> w1{(T)0, (T)0}, w2[W2];
+        // the tile's t2 values go to the group's two buffers in turn: slower warps of
+        // the group may still read the other one for the tile before
+        cpx<T> *const t2s = t2b + (i / NG & 1) * Cfg::T2;
+        cpx<T> w1{(T)0, (T)0};
         if constexpr (TWM != 0) {
             const unsigned f = TWM == 3 ? (unsigned)(active ? col : 0) : (unsigned)b;
-            w1 = ldg_c(t1 + f * (unsigned)t);
+            w1 = ldg_c(t1 + f * (unsigned)G + t);
 #pragma unroll
             for (int j = 0; j < W2; j++)
-                if (W2 * GT == Cfg::T2 || tid + j * GT < Cfg::T2) w2[j] = ldg_c(t2 + f * (unsigned)(t + j * G));
+                if (W2 * GT == Cfg::T2 || tid + j * GT < Cfg::T2) cp_async8(t2s + tid + j * GT, t2 + f * (unsigned)E + (t + j * G));
         }
         const bool ok = stage_wait(&full[buf], &seq[buf], i, par);
-        cpx<T> *const S = stage0 + (size_t)buf * Cfg::STAGE;
         cpx<T> v[E];
 #pragma unroll
         for (int q = 0; q < E; q++) {
@@ -252,30 +288,14 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU 
         stockham_run<T, LOGL, E_, INV, TwShared>(
             v, t, [my](int k) -> cpx<T> & { return my[Cfg::padded(k)]; }, tws, [bar]() { bar_group(bar, GT); },
             [&]() {
-                // the stage is free once the whole group has read it; only
-                // the issuing warp waits for that
-                if (tid < 32) {
-                    bar_group(bar + 1, GT);
-                    if (tid == 0) {
-                        fence_proxy_async_smem();
-                        if (landed) issue(i + NB);
-                    }
-                    __syncwarp();
-                } else {
-                    bar_group_arrive(bar + 1, GT);
-                }
+                stage_read(bar + 1, GT, tid);
+                if (!late) stage_refill(bar + 1, GT, tid, landed, i + NB, issue);
             },
             [&]() {
                 // every thread of the group holds its inputs: the stage
                 // takes the exchange
+                if constexpr (TWM != 0) cp_async_wait();
                 landed = bar_group_and(bar, GT, ok);
-                if constexpr (TWM != 0) {
-                    // (read after the exchange barrier, overwritten after the
-                    // next tile's first barrier)
-#pragma unroll
-                    for (int j = 0; j < W2; j++)
-                        if (W2 * GT == Cfg::T2 || tid + j * GT < Cfg::T2) t2s[tid + j * GT] = w2[j];
-                }
             });
         if (!landed) return false;
         if (active) {
@@ -291,6 +311,7 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU 
                 }
             }
         }
+        if (late) stage_refill(bar + 1, GT, tid, landed, i + NB, issue);
         return true;
     });
 }
@@ -302,7 +323,7 @@ template <typename T, int LOGL, int C, int E_, int NG, int NB, bool INV>
 __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, LAND_ROW>::THREADS, 1)
     k_rowpass_tma(const cpx<T> *__restrict__ in, cpx<T> *__restrict__ out, long long nrows, long long ld_in,
               long long ostride, long long idist, long long odist, long long nbatch, const cpx<T> *__restrict__ tw,
-              unsigned *err, T scale)
+              unsigned *err, T scale, unsigned late)
 {
     using Cfg = PipeCfg<T, LOGL, C, E_, NG, NB, LAND_ROW>;
     using SP = typename Cfg::SP;
@@ -312,7 +333,6 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, LAND_ROW>::THR
     cpx<T> *const tws = stage0 + (size_t)NB * Cfg::STAGE;
     uint64_t *const full = reinterpret_cast<uint64_t *>(smem_raw + Cfg::BAR_OFF);
     int *const seq = reinterpret_cast<int *>(full + NB);
-
     const int grp = threadIdx.x / GT, tid = threadIdx.x - grp * GT;
     const int bar = 1 + 2 * grp;
     // a half-warp takes at most 8 rows (Cfg::CB) and 16 / CB values of t
@@ -336,20 +356,21 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, LAND_ROW>::THR
         const int w = w0 + i * step;
         if (w >= total) return;
         const int buf = i % NB;
+        cpx<T> *const S = stage0 + (size_t)buf * Cfg::STAGE;
         const int b = (int)((unsigned)w / (unsigned)tiles), row0 = (w - b * tiles) * C;
         const int rows = (int)(nrows - row0 < C ? nrows - row0 : C);
         mbar_arrive_expect_tx(&full[buf], (uint32_t)(rows * N * sizeof(cpx<T>)));
         seq_publish(&seq[buf], i);
         const cpx<T> *src = in + (long long)b * idist + (long long)row0 * ld_in;
         for (int r = 0; r < rows; r++)
-            bulk_load(stage0 + (size_t)buf * Cfg::STAGE + r * Cfg::RP, src + r * ld_in, N * sizeof(cpx<T>), &full[buf]);
+            bulk_load(S + r * Cfg::RP, src + r * ld_in, N * sizeof(cpx<T>), &full[buf]);
     };
     pipe_loop<Cfg>(full, seq, err, w0, step, total, issue, [&](int i, int buf, uint32_t par) {
         const int w = w0 + i * step;
+        cpx<T> *const S = stage0 + (size_t)buf * Cfg::STAGE;
         const int wb = (int)((unsigned)w / (unsigned)tiles);
         const long long b = wb, row = (long long)(w - wb * tiles) * C + s;
         const bool ok = stage_wait(&full[buf], &seq[buf], i, par);
-        cpx<T> *const S = stage0 + (size_t)buf * Cfg::STAGE;
         cpx<T> v[E];
 #pragma unroll
         for (int q = 0; q < E; q++) v[q] = S[s * Cfg::RP + t + q * G];
@@ -358,16 +379,8 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, LAND_ROW>::THR
         stockham_run<T, LOGL, E_, INV, TwShared>(
             v, t, [my](int k) -> cpx<T> & { return my[Cfg::padded(k)]; }, tws, [bar]() { bar_group(bar, GT); },
             [&]() {
-                if (tid < 32) {
-                    bar_group(bar + 1, GT);
-                    if (tid == 0) {
-                        fence_proxy_async_smem();
-                        if (landed) issue(i + NB);
-                    }
-                    __syncwarp();
-                } else {
-                    bar_group_arrive(bar + 1, GT);
-                }
+                stage_read(bar + 1, GT, tid);
+                if (!late) stage_refill(bar + 1, GT, tid, landed, i + NB, issue);
             },
             [&]() { landed = bar_group_and(bar, GT, ok); });
         if (!landed) return false;
@@ -377,6 +390,7 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, LAND_ROW>::THR
 #pragma unroll
             for (int q = 0; q < E; q++, dst += st) stcs_c(dst, scl(v[q], scale));
         }
+        if (late) stage_refill(bar + 1, GT, tid, landed, i + NB, issue);
         return true;
     });
 }

@@ -54,15 +54,18 @@ const TileKernel *tile_find(int dtype, int variant, int logl, int c);
 // widest registered column count <= max_c (0 if none)
 int tile_widest(int dtype, int variant, int logl, int max_c);
 
+// late (tiles_pipe.cuh): each stage is refilled after its tile's stores
 // Launch over tiles x nbatch CTAs (the batch is split into launches of at
 // most 65535 items).  Strides and distances are in complex elements.
 cudaError_t launch_colpass(const TileKernel &k, int inverse, long long tiles, long long nbatch,
                            const void *in, void *out, long long ncols, long long ld_in, long long ld_out,
                            long long idist, long long odist, const void *tw, const void *tw_lo,
-                           const void *tw_hi, int lo_bits, unsigned nmask, cudaStream_t st, double scale = 1.0);
+                           const void *tw_hi, int lo_bits, unsigned nmask, cudaStream_t st, double scale = 1.0,
+                           bool late = false);
 cudaError_t launch_rowpass(const TileKernel &k, int inverse, long long tiles, long long nbatch,
                            const void *in, void *out, long long nrows, long long ld_in, long long ostride,
-                           long long idist, long long odist, const void *tw, cudaStream_t st, double scale = 1.0);
+                           long long idist, long long odist, const void *tw, cudaStream_t st, double scale = 1.0,
+                           bool late = false);
 
 // 3D tiled tensor map over 8-byte units (dims x, y, z; byte strides of y
 // and z; box bx x by x 1); false if the driver entry point is missing or
@@ -70,6 +73,9 @@ cudaError_t launch_rowpass(const TileKernel &k, int inverse, long long tiles, lo
 bool make_tensor_map_3d(CUtensorMap *map, const void *base, unsigned long long dx, unsigned long long dy,
                         unsigned long long dz, unsigned long long sy_bytes, unsigned long long sz_bytes, unsigned bx,
                         unsigned by);
+
+// SMs of the current device
+int sm_count();
 
 // the device error word the persistent kernels report timeouts into
 unsigned *device_error_word();
