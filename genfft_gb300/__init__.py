@@ -13,6 +13,13 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
+from collections import OrderedDict
+
+try:
+    import torch
+except ImportError:  # the ABI itself needs no torch; the tensor functions below do
+    torch = None
 
 __all__ = ["GFFTError", "Plan", "lib", "lib_path", "fft", "fft_tc", "ifft", "fft_no_scramble", "rfft", "fft_real_input",
            "fft_interleave", "separate_2x", "dit", "fft_vert", "fft_vert_no_scramble", "fft2", "rfft2",
@@ -117,19 +124,30 @@ def _check(status: int) -> None:
         raise GFFTError(status, msg.decode() if msg else "")
 
 
+# the current stream's handle without a Stream object around it (0.1 us
+# against 2.9)
+_raw_stream = getattr(getattr(torch, "_C", None), "_cuda_getCurrentRawStream", None)
+
+
 def _stream_ptr(stream=None) -> int:
-    import torch
-    s = torch.cuda.current_stream() if stream is None else stream
-    return s.cuda_stream
+    if stream is not None:
+        return stream.cuda_stream
+    if _raw_stream is not None:
+        return _raw_stream(torch.cuda.current_device())
+    return torch.cuda.current_stream().cuda_stream
+
+
+_CODES = {} if torch is None else {torch.complex64: F32, torch.float32: F32, torch.complex128: F64,
+                                   torch.float64: F64}
+_COMPLEX = () if torch is None else (torch.complex64, torch.complex128)
+_REAL = () if torch is None else (torch.float32, torch.float64)
 
 
 def _dtype_code(t) -> int:
-    import torch
-    if t.dtype in (torch.complex64, torch.float32):
-        return F32
-    if t.dtype in (torch.complex128, torch.float64):
-        return F64
-    raise TypeError(f"unsupported dtype {t.dtype}")
+    code = _CODES.get(t.dtype)
+    if code is None:
+        raise TypeError(f"unsupported dtype {t.dtype}")
+    return code
 
 
 class Plan:
@@ -187,6 +205,32 @@ class Plan:
             pass
 
 
+# Plans of the functions below that make one a call.  Only plans without a
+# workspace are kept: their execs touch nothing but their arguments and the
+# process-wide tables, so any thread and stream may run one at any time.
+_STATELESS: "OrderedDict[tuple, Plan]" = OrderedDict()
+_STATELESS_MAX = 64
+_stateless_mu = threading.Lock()
+
+
+def _call_plan(*args) -> Plan:
+    key = (torch.cuda.current_device(), *args)
+    with _stateless_mu:
+        p = _STATELESS.get(key)
+        if p is not None:
+            _STATELESS.move_to_end(key)
+            return p
+    p = Plan(*args)
+    size = ctypes.c_size_t()
+    _check(lib().gfft_plan_workspace_size(p.handle, ctypes.byref(size)))
+    if size.value == 0:
+        with _stateless_mu:
+            _STATELESS[key] = p
+            if len(_STATELESS) > _STATELESS_MAX:
+                _STATELESS.popitem(last=False)
+    return p
+
+
 def max_fused_size(dtype: int = F32) -> int:
     """Largest n one fused single-kernel transform handles for dtype."""
     return int(lib().gfft_max_fused_size(dtype))
@@ -211,9 +255,8 @@ def _check_cuda_tensor(x, name="x"):
 def fft(x, inverse: bool = False, out=None):
     """Batched C2C over the last dimension (FFT<T>::transform<inv>, fft.h:80-85).
     The inverse is unscaled."""
-    import torch
     _check_cuda_tensor(x)
-    if x.dtype not in (torch.complex64, torch.complex128):
+    if x.dtype not in _COMPLEX:
         raise TypeError("fft expects complex64/complex128")
     n = x.shape[-1]
     batch = x.numel() // n if n else 0
@@ -231,7 +274,6 @@ def fft_tc(x, inverse: bool = False, mode: int = MODE_TC_FP16, out=None):
     """Batched fp32 C2C over the last dimension (n = 256, 4096 or 65536) on
     the split-precision tensor-core path (mode MODE_TC_FP16 or MODE_TC_BF16).
     Same conventions as fft(): unscaled inverse."""
-    import torch
     _check_cuda_tensor(x)
     if x.dtype != torch.complex64:
         raise TypeError("fft_tc expects complex64")
@@ -252,7 +294,6 @@ def ifft(x, out=None):
 
 
 def _cdtype_for_real(x):
-    import torch
     return torch.complex64 if x.dtype == torch.float32 else torch.complex128
 
 
@@ -269,23 +310,21 @@ def fft_no_scramble(x, inverse: bool = False):
 def rfft(x, half: bool = True, out=None):
     """RealFFT<T>::forward over the last dimension (FFTReal.h:204-213):
     n reals -> n/2+1 bins (half) or the full Hermitian n bins."""
-    import torch
     _check_cuda_tensor(x)
-    if x.dtype not in (torch.float32, torch.float64):
+    if x.dtype not in _REAL:
         raise TypeError("rfft expects float32/float64")
     n = x.shape[-1]
     batch = x.numel() // n
     m = n // 2 + 1 if half else n
     if out is None:
         out = torch.empty(*x.shape[:-1], m, dtype=_cdtype_for_real(x), device=x.device)
-    p = Plan(KIND_R2C, _dtype_code(x), n, 0, batch, FLAG_HALF_SPECTRUM if half else 0, 0, n, 0, m)
+    p = _call_plan(KIND_R2C, _dtype_code(x), n, 0, batch, FLAG_HALF_SPECTRUM if half else 0, 0, n, 0, m)
     p.exec(out, x)
     return out
 
 
 def fft_real_input(x):
     """FFT<T>::transform_real (fft.h:90-94): full complex spectrum of reals."""
-    import torch
     _check_cuda_tensor(x)
     n = x.shape[-1]
     out = torch.empty(*x.shape, dtype=_cdtype_for_real(x), device=x.device)
@@ -296,7 +335,6 @@ def fft_real_input(x):
 
 def fft_interleave(a, b):
     """FFT<T>::transform_interleave (fft.h:100-105): FFT of a + i b (1D)."""
-    import torch
     _check_cuda_tensor(a, "a")
     _check_cuda_tensor(b, "b")
     n = a.shape[-1]
@@ -308,7 +346,6 @@ def fft_interleave(a, b):
 
 def separate_2x(z):
     """separate_2x_real_FFT (FFTReal.h:34-66) -> (X, Y)."""
-    import torch
     _check_cuda_tensor(z, "z")
     n = z.shape[-1]
     a, b = torch.empty_like(z), torch.empty_like(z)
@@ -320,7 +357,6 @@ def separate_2x(z):
 def dit(z, n: int, half: bool):
     """DIT<T>(n).apply on an n/2-point spectrum z (fft.h:180-188); returns
     an n-element buffer (only n/2+1 written when half)."""
-    import torch
     _check_cuda_tensor(z, "z")
     out = torch.zeros(n, dtype=z.dtype, device=z.device)
     buf = torch.zeros(n, dtype=z.dtype, device=z.device)
@@ -331,7 +367,6 @@ def dit(z, n: int, half: bool):
 
 def fft_vert(x, inverse: bool = False, out=None):
     """FFTVert<T>(rows).transform on an [rows, cols] tensor (fft.h:145-150)."""
-    import torch
     _check_cuda_tensor(x)
     rows, cols = x.shape
     if out is None:
@@ -353,13 +388,12 @@ def fft_vert_no_scramble(x, inverse: bool = False):
 def fft2(x, inverse: bool = False, out=None):
     """FFT2D<T>(W, H).transform on [..., H, W] (fft.h:213-218); batched over
     leading dimensions through a plan."""
-    import torch
     _check_cuda_tensor(x)
     H, W = x.shape[-2:]
     batch = x.numel() // (H * W)
     if out is None:
         out = torch.empty_like(x)
-    p = Plan(KIND_C2C_2D, _dtype_code(x), W, H, batch)
+    p = _call_plan(KIND_C2C_2D, _dtype_code(x), W, H, batch)
     p.exec(out, x, inverse)
     return out
 
@@ -367,21 +401,19 @@ def fft2(x, inverse: bool = False, out=None):
 def rfft2(x, half: bool = False, out=None):
     """RealFFT2D<T>(W, H).forward on [..., H, W] reals (FFTReal.h:83-104):
     full-width Hermitian [H, W] output, or [H, W/2+1] when half."""
-    import torch
     _check_cuda_tensor(x)
     H, W = x.shape[-2:]
     batch = x.numel() // (H * W)
     m = W // 2 + 1 if half else W
     if out is None:
         out = torch.empty(*x.shape[:-1], m, dtype=_cdtype_for_real(x), device=x.device)
-    p = Plan(KIND_R2C_2D, _dtype_code(x), W, H, batch, FLAG_HALF_SPECTRUM if half else 0, W, H * W, m, H * m)
+    p = _call_plan(KIND_R2C_2D, _dtype_code(x), W, H, batch, FLAG_HALF_SPECTRUM if half else 0, W, H * W, m, H * m)
     p.exec(out, x)
     return out
 
 
 def rfft2_2x(a, b):
     """RealFFT2D<T>::forward_2x (FFTReal.h:114-118): 2D FFT of a + i b."""
-    import torch
     _check_cuda_tensor(a, "a")
     _check_cuda_tensor(b, "b")
     H, W = a.shape

@@ -24,6 +24,7 @@ import math
 from collections import OrderedDict
 
 import torch
+import torch.autograd.forward_ad as _forward_ad
 
 from . import (F32, F64, FLAG_HALF_SPECTRUM, KIND_C2C, KIND_C2C_2D, KIND_R2C, KIND_R2C_2D, KIND_VERT,
                Plan)
@@ -33,6 +34,8 @@ __all__ = ["fft", "ifft", "rfft", "irfft", "fft2", "ifft2", "rfft2", "irfft2", "
 _NORMS = (None, "backward", "forward", "ortho")
 _PLANS: "OrderedDict[tuple, Plan]" = OrderedDict()
 _MAX_PLANS = 64
+# whether a functorch transform is active (taken to be so where torch cannot say)
+_functorch_active = getattr(torch._C, "_are_functorch_transforms_active", lambda: True)
 
 
 def norm_scale(norm, n: int, inverse: bool) -> float:
@@ -102,60 +105,65 @@ def _resize(x, n: int, dim: int):
 # ---------------------------------------------------------------------------
 # differentiable kernels (last dimension, or last two for 2D)
 
+def _c2c(x, inverse: bool, scale: float):
+    x = x.contiguous()
+    n = x.shape[-1]
+    p = _plan(KIND_C2C, _code(x), n, 0, x.numel() // n)
+    return p.exec(torch.empty_like(x), x, inverse, scale=scale)
+
+
+def _c2c2d(x, inverse: bool, scale: float):
+    x = x.contiguous()
+    h, w = x.shape[-2], x.shape[-1]
+    p = _plan(KIND_C2C_2D, _code(x), w, h, x.numel() // (h * w))
+    return p.exec(torch.empty_like(x), x, inverse, scale=scale)
+
+
+def _r2c(x, scale: float):
+    x = x.contiguous()
+    n = x.shape[-1]
+    p = _plan(KIND_R2C, _code(x), n, 0, x.numel() // n, FLAG_HALF_SPECTRUM)
+    cdt = torch.complex128 if x.dtype == torch.float64 else torch.complex64
+    y = torch.empty(*x.shape[:-1], n // 2 + 1, dtype=cdt, device=x.device)
+    return p.exec(y, x, False, scale=scale)
+
+
+def _c2r(y, n: int, scale: float):
+    y = y.contiguous()
+    p = _plan(KIND_R2C, _code(y), n, 0, y.numel() // y.shape[-1], FLAG_HALF_SPECTRUM)
+    rdt = torch.float64 if y.dtype == torch.complex128 else torch.float32
+    x = torch.empty(*y.shape[:-1], n, dtype=rdt, device=y.device)
+    return p.exec(x, y, True, scale=scale)
+
+
 class _C2C(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, inverse: bool, scale: float):
-        x = x.contiguous()
-        n = x.shape[-1]
-        p = _plan(KIND_C2C, _code(x), n, 0, x.numel() // n)
-        y = torch.empty_like(x)
-        p.exec(y, x, inverse, scale=scale)
         ctx.inverse, ctx.scale = inverse, scale
-        return y
+        return _c2c(x, inverse, scale)
 
     @staticmethod
     def backward(ctx, g):
         # (s F)^H = s F^H: the conjugate-direction transform, same scale
-        g = g.contiguous()
-        n = g.shape[-1]
-        p = _plan(KIND_C2C, _code(g), n, 0, g.numel() // n)
-        gx = torch.empty_like(g)
-        p.exec(gx, g, not ctx.inverse, scale=ctx.scale)
-        return gx, None, None
+        return _c2c(g, not ctx.inverse, ctx.scale), None, None
 
 
 class _C2C2D(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, inverse: bool, scale: float):
-        x = x.contiguous()
-        h, w = x.shape[-2], x.shape[-1]
-        p = _plan(KIND_C2C_2D, _code(x), w, h, x.numel() // (h * w))
-        y = torch.empty_like(x)
-        p.exec(y, x, inverse, scale=scale)
         ctx.inverse, ctx.scale = inverse, scale
-        return y
+        return _c2c2d(x, inverse, scale)
 
     @staticmethod
     def backward(ctx, g):
-        g = g.contiguous()
-        h, w = g.shape[-2], g.shape[-1]
-        p = _plan(KIND_C2C_2D, _code(g), w, h, g.numel() // (h * w))
-        gx = torch.empty_like(g)
-        p.exec(gx, g, not ctx.inverse, scale=ctx.scale)
-        return gx, None, None
+        return _c2c2d(g, not ctx.inverse, ctx.scale), None, None
 
 
 class _R2C(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, scale: float):
-        x = x.contiguous()
-        n = x.shape[-1]
-        p = _plan(KIND_R2C, _code(x), n, 0, x.numel() // n, FLAG_HALF_SPECTRUM)
-        cdt = torch.complex128 if x.dtype == torch.float64 else torch.complex64
-        y = torch.empty(*x.shape[:-1], n // 2 + 1, dtype=cdt, device=x.device)
-        p.exec(y, x, False, scale=scale)
-        ctx.n, ctx.scale = n, scale
-        return y
+        ctx.n, ctx.scale = x.shape[-1], scale
+        return _r2c(x, scale)
 
     @staticmethod
     def backward(ctx, g):
@@ -171,13 +179,8 @@ class _R2C(torch.autograd.Function):
 class _C2R(torch.autograd.Function):
     @staticmethod
     def forward(ctx, y, n: int, scale: float):
-        y = y.contiguous()
-        p = _plan(KIND_R2C, _code(y), n, 0, y.numel() // y.shape[-1], FLAG_HALF_SPECTRUM)
-        rdt = torch.float64 if y.dtype == torch.complex128 else torch.float32
-        x = torch.empty(*y.shape[:-1], n, dtype=rdt, device=y.device)
-        p.exec(x, y, True, scale=scale)
         ctx.n, ctx.scale = n, scale
-        return x
+        return _c2r(y, n, scale)
 
     @staticmethod
     def backward(ctx, g):
@@ -188,6 +191,34 @@ class _C2R(torch.autograd.Function):
         gy = torch.empty(*g.shape[:-1], n // 2 + 1, dtype=cdt, device=g.device)
         p.adjoint(gy, g, True)
         return (gy.mul_(ctx.scale) if ctx.scale != 1.0 else gy), None, None
+
+
+def _plain(x) -> bool:
+    """Whether the transform of x is nobody's business but its caller's: an
+    ordinary tensor outside autograd, forward-mode differentiation and the
+    function transforms (vmap, grad, ...).  Such calls skip the
+    autograd.Function around the kernel (10 us a call); every other one goes
+    through it and gets its results, or its errors."""
+    return (type(x) is torch.Tensor and not (x.requires_grad and torch.is_grad_enabled())
+            and _forward_ad._current_level < 0 and not _functorch_active())
+
+
+def _last(x, d: int):
+    """Dimension d moved to the end."""
+    return x if d == x.dim() - 1 else x.movedim(d, -1)
+
+
+def _back(y, d: int):
+    return y if d == y.dim() - 1 else y.movedim(-1, d)
+
+
+def _last2(x, d0: int, d1: int):
+    """Dimensions (d0, d1) moved to the end."""
+    return x if (d0, d1) == (x.dim() - 2, x.dim() - 1) else x.movedim((d0, d1), (-2, -1))
+
+
+def _back2(y, d0: int, d1: int):
+    return y if (d0, d1) == (y.dim() - 2, y.dim() - 1) else y.movedim((-2, -1), (d0, d1))
 
 
 # ---------------------------------------------------------------------------
@@ -206,16 +237,16 @@ def fft(input, n=None, dim=-1, norm=None):
     """torch.fft.fft for power-of-two n."""
     x, d = _one_dim(input, n, dim, True)
     _check_pow2(x.shape[d], "n")
-    y = _C2C.apply(x.movedim(d, -1), False, norm_scale(norm, x.shape[d], False))
-    return y.movedim(-1, d)
+    f = _c2c if _plain(x) else _C2C.apply
+    return _back(f(_last(x, d), False, norm_scale(norm, x.shape[d], False)), d)
 
 
 def ifft(input, n=None, dim=-1, norm=None):
     """torch.fft.ifft for power-of-two n."""
     x, d = _one_dim(input, n, dim, True)
     _check_pow2(x.shape[d], "n")
-    y = _C2C.apply(x.movedim(d, -1), True, norm_scale(norm, x.shape[d], True))
-    return y.movedim(-1, d)
+    f = _c2c if _plain(x) else _C2C.apply
+    return _back(f(_last(x, d), True, norm_scale(norm, x.shape[d], True)), d)
 
 
 def rfft(input, n=None, dim=-1, norm=None):
@@ -225,8 +256,8 @@ def rfft(input, n=None, dim=-1, norm=None):
     if n is not None:
         x = _resize(x, n, d)
     _check_pow2(x.shape[d], "n")
-    y = _R2C.apply(x.movedim(d, -1), norm_scale(norm, x.shape[d], False))
-    return y.movedim(-1, d)
+    f = _r2c if _plain(x) else _R2C.apply
+    return _back(f(_last(x, d), norm_scale(norm, x.shape[d], False)), d)
 
 
 def irfft(input, n=None, dim=-1, norm=None):
@@ -237,8 +268,8 @@ def irfft(input, n=None, dim=-1, norm=None):
     n = 2 * (y.shape[d] - 1) if n is None else n
     _check_pow2(n, "n")
     y = _resize(y, n // 2 + 1, d)
-    x = _C2R.apply(y.movedim(d, -1), n, norm_scale(norm, n, True))
-    return x.movedim(-1, d)
+    f = _c2r if _plain(y) else _C2R.apply
+    return _back(f(_last(y, d), n, norm_scale(norm, n, True)), d)
 
 
 def _two_dims(x, s, dim):
@@ -258,8 +289,8 @@ def fft2(input, s=None, dim=(-2, -1), norm=None):
     h, w = x.shape[d0], x.shape[d1]
     _check_pow2(h, "s[0]")
     _check_pow2(w, "s[1]")
-    y = _C2C2D.apply(x.movedim((d0, d1), (-2, -1)), False, norm_scale(norm, h * w, False))
-    return y.movedim((-2, -1), (d0, d1))
+    f = _c2c2d if _plain(x) else _C2C2D.apply
+    return _back2(f(_last2(x, d0, d1), False, norm_scale(norm, h * w, False)), d0, d1)
 
 
 def ifft2(input, s=None, dim=(-2, -1), norm=None):
@@ -268,8 +299,8 @@ def ifft2(input, s=None, dim=(-2, -1), norm=None):
     h, w = x.shape[d0], x.shape[d1]
     _check_pow2(h, "s[0]")
     _check_pow2(w, "s[1]")
-    y = _C2C2D.apply(x.movedim((d0, d1), (-2, -1)), True, norm_scale(norm, h * w, True))
-    return y.movedim((-2, -1), (d0, d1))
+    f = _c2c2d if _plain(x) else _C2C2D.apply
+    return _back2(f(_last2(x, d0, d1), True, norm_scale(norm, h * w, True)), d0, d1)
 
 
 def _no_grad(x, name):
@@ -285,13 +316,13 @@ def rfft2(input, s=None, dim=(-2, -1), norm=None):
     h, w = x.shape[d0], x.shape[d1]
     _check_pow2(h, "s[0]")
     _check_pow2(w, "s[1]")
-    x = x.movedim((d0, d1), (-2, -1)).contiguous()
+    x = _last2(x, d0, d1).contiguous()
     batch = x.numel() // (h * w)
     p = _plan(KIND_R2C_2D, _code(x), w, h, batch, FLAG_HALF_SPECTRUM)
     cdt = torch.complex128 if x.dtype == torch.float64 else torch.complex64
     y = torch.empty(*x.shape[:-1], w // 2 + 1, dtype=cdt, device=x.device)
     p.exec(y, x, False, scale=norm_scale(norm, h * w, False))
-    return y.movedim((-2, -1), (d0, d1))
+    return _back2(y, d0, d1)
 
 
 def irfft2(input, s=None, dim=(-2, -1), norm=None):
@@ -308,7 +339,7 @@ def irfft2(input, s=None, dim=(-2, -1), norm=None):
     _check_pow2(h, "s[0]")
     _check_pow2(w, "s[1]")
     m = w // 2 + 1
-    y = _resize(_resize(y, h, d0), m, d1).movedim((d0, d1), (-2, -1)).contiguous()
+    y = _last2(_resize(_resize(y, h, d0), m, d1), d0, d1).contiguous()
     batch = y.numel() // (h * m)
     cols = _plan(KIND_VERT, _code(y), h, m, batch)
     t = torch.empty_like(y)
@@ -317,4 +348,4 @@ def irfft2(input, s=None, dim=(-2, -1), norm=None):
     rdt = torch.float64 if y.dtype == torch.complex128 else torch.float32
     x = torch.empty(*y.shape[:-1], w, dtype=rdt, device=y.device)
     rows.exec(x, t, True, scale=norm_scale(norm, h * w, True))
-    return x.movedim((-2, -1), (d0, d1))
+    return _back2(x, d0, d1)
