@@ -253,6 +253,7 @@ static void check_ptr(const void *ptr, size_t align, const char *name)
 // per-call layout (reference-shaped entry points override the plan's)
 struct Layout {
     long long batch, istride, idist, ostride, odist;
+    bool host = false;  // C2C on host memory (exec_host's direct way)
 };
 
 static Layout plan_layout(const gfft_plan_s &p)
@@ -292,7 +293,7 @@ static void exec_body(gfft_plan_s &p, int inverse, void *out, const void *in, co
         } else if (d.mode != GFFT_MODE_PLAIN) {
             p.tc.run(inverse, in, out, L.batch, L.idist, L.odist, L.istride, L.ostride, st, scale);
         } else {
-            p.c2c.run(inverse, in, out, L.batch, L.idist, L.odist, L.istride, L.ostride, st, scale);
+            p.c2c.run(inverse, in, out, L.batch, L.idist, L.odist, L.istride, L.ostride, st, scale, L.host);
         }
         break;
     case GFFT_KIND_R2C: {
@@ -545,7 +546,9 @@ static void exec_host(gfft_plan_s &p, int inverse, void *out, const void *in)
                 check_cuda(cudaEventCreateWithFlags(&p.ev_done[i], cudaEventDisableTiming), "event");
             }
         }
-        exec_plan(p, inverse, out, in, plan_layout(p), p.compute_stream);
+        Layout L = plan_layout(p);
+        L.host = true;
+        exec_plan(p, inverse, out, in, L, p.compute_stream);
         check_cuda(cudaStreamSynchronize(p.compute_stream), "sync");
         return;
     }

@@ -31,13 +31,28 @@ struct FusedC2CArgs {
     long long idist, odist;       // elements between transforms
     long long istride, ostride;   // elements between points
     const void *tw;               // device twiddle table for (dtype, logn)
+    const void *tw_tma = nullptr; // that of the persistent version, if there is one
     double scale = 1.0;           // applied to every output (norm= scaling)
+    bool host = false;            // in / out are host memory the kernel reaches over the link
 };
 int fused_max_logn(int dtype);
 size_t fused_twiddle_count(int dtype, int logn);              // complex elements
 void fused_twiddle_fill(int dtype, int logn, void *host_buf);  // writes that many
 cudaError_t launch_fused_c2c(int dtype, int logn, int inverse, const FusedC2CArgs &a,
                              cudaStream_t st);
+
+// ---- the persistent versions for fp32, complex lengths 2^12 .. 2^14
+// (fused_tma.cu): many transforms of dense, 16-byte aligned input ----------
+constexpr int FUSED_TMA_MIN = 12, FUSED_TMA_MAX = 14;
+size_t fused_tma_twiddle_count(int logn);
+void fused_tma_twiddle_fill(int logn, void *host_buf);
+bool fused_tma_takes(int logn, bool real, long long batch);
+cudaError_t launch_fused_tma_c2c(int logn, int inverse, const FusedC2CArgs &a, cudaStream_t st);
+// distances in complex elements; x2 / half: interior bins doubled / halved
+cudaError_t launch_fused_tma_r2c(int logh, bool x2, const void *in, void *out, long long batch, long long idist,
+                                 long long odist, const void *tw, const void *dtw, cudaStream_t st, double scale);
+cudaError_t launch_fused_tma_c2r(int logh, bool half, const void *in, void *out, long long batch, long long idist,
+                                 long long odist, const void *tw, const void *dtw, cudaStream_t st, double scale);
 
 // Opts fn in to `smem` bytes of dynamic shared memory when that is above
 // the 48 KB default, once per (device, function).

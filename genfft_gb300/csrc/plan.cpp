@@ -3,7 +3,8 @@
 //
 // Path per size (the defaults, each measured on GB300; the environment
 // knobs read below override them):
-//   C2C  n <= 2^14 (fp32) / 2^13 (fp64)  one fused kernel (c2c_fused.cu)
+//   C2C  n <= 2^14 (fp32) / 2^13 (fp64)  one fused kernel (c2c_fused.cu; many
+//                                        fp32 2^12 .. 2^14: fused_tma.cu)
 //        fp32 2^16                       the persistent four-step kernel
 //                                        (fourstep.cuh), one launch a batch
 //        fp32 2^17 .. 2^24               column + row launches of the
@@ -88,6 +89,14 @@ static const void *tile_table(int dtype, const TileKernel *k, int logl, int c)
                         dtype, k->twcount, [k](void *buf) { k->fill(buf); });
 }
 
+// the Stockham table of the persistent fused kernels (fused_tma.cu), or null
+static const void *fused_tma_table(int dtype, int logn)
+{
+    if (dtype != GFFT_F32 || logn < FUSED_TMA_MIN || logn > FUSED_TMA_MAX) return nullptr;
+    return cached_table("fusedtma/" + std::to_string(logn), dtype, fused_tma_twiddle_count(logn),
+                        [logn](void *buf) { fused_tma_twiddle_fill(logn, buf); });
+}
+
 // ---------------------------------------------------------------------------
 // C2C
 
@@ -100,6 +109,7 @@ void C2CCore::init(int dtype_, int logn_, long long batch_hint, int path, bool r
         const int d = dtype, l = logn;
         tw = cached_table("fused/" + std::to_string(d) + "/" + std::to_string(l), d, fused_twiddle_count(d, l),
                           [d, l](void *buf) { fused_twiddle_fill(d, l, buf); });
+        tw_tma = fused_tma_table(dtype, logn);
         return;
     }
     if (logn > 24) fail(GFFT_ERR_INVALID_SIZE, "transform length above 2^24 is not supported");
@@ -279,10 +289,10 @@ int C2CCore::launches(long long batch) const
 }
 
 void C2CCore::run(int inverse, const void *in, void *out, long long batch, long long idist, long long odist,
-                  long long istride, long long ostride, cudaStream_t st, double scale) const
+                  long long istride, long long ostride, cudaStream_t st, double scale, bool host) const
 {
     if (algo == 1) {
-        FusedC2CArgs a{in, out, batch, idist, odist, istride, ostride, tw, scale};
+        FusedC2CArgs a{in, out, batch, idist, odist, istride, ostride, tw, tw_tma, scale, host};
         check_cuda(launch_fused_c2c(dtype, logn, inverse, a, st), "launch fused C2C");
         return;
     }
@@ -559,6 +569,7 @@ void R2CCore::init(int dtype_, int logn_, int half_, long long batch_hint)
         algo = 1;
         tw = cached_table("r2c/" + std::to_string(d) + "/" + std::to_string(lh), d, r2c_twiddle_count(d, lh),
                           [d, lh](void *buf) { r2c_twiddle_fill(d, lh, buf); });
+        tw_tma = fused_tma_table(dtype, lh);
         return;
     }
     // pipelined passes (real_pipe.cu): rows of 2^9, columns of 2^8 .. 2^12
@@ -615,6 +626,10 @@ void R2CCore::run(const void *in, void *out, long long batch, long long idist, l
     if (mode < 0) mode = half ? 0 : 1;
     if (algo == 0) {
         check_cuda(launch_r2c_one(dtype, in, out, batch, idist, odist, st, scale), "launch R2C n=1");
+    } else if (algo == 1 && tw_tma && mode != 1 && ((uintptr_t)in & 15u) == 0 && idist % 4 == 0 &&
+               fused_tma_takes(logn - 1, true, batch)) {
+        check_cuda(launch_fused_tma_r2c(logn - 1, mode == 2, in, out, batch, idist / 2, odist, tw_tma, dtw, st, scale),
+                   "launch persistent fused R2C");
     } else if (algo == 1) {
         check_cuda(launch_r2c_fused(dtype, logn - 1, mode, in, out, batch, idist, odist, tw, dtw, st, scale),
                    "launch fused R2C");
@@ -670,6 +685,7 @@ void C2RCore::init(int dtype_, int logn_, long long batch_hint)
         algo = 1;
         tw = cached_table("r2c/" + std::to_string(d) + "/" + std::to_string(lh), d, r2c_twiddle_count(d, lh),
                           [d, lh](void *buf) { r2c_twiddle_fill(d, lh, buf); });
+        tw_tma = fused_tma_table(dtype, lh);
         if (!c2r_fused_fits(dtype, lh, 2)) {
             fold_split = true;
             c2c.init(dtype, lh, batch_hint);
@@ -699,6 +715,9 @@ void C2RCore::run(const void *in, void *out, long long batch, long long idist, l
 {
     if (algo == 0) {
         check_cuda(launch_c2r_one(dtype, in, out, batch, idist, odist, st, scale), "launch C2R n=1");
+    } else if (algo == 1 && tw_tma && wmode != 2 && fused_tma_takes(logn - 1, true, batch)) {
+        check_cuda(launch_fused_tma_c2r(logn - 1, wmode == 1, in, out, batch, idist, odist / 2, tw_tma, dtw, st, scale),
+                   "launch persistent fused C2R");
     } else if (algo == 1 && !(fold_split && wmode == 2)) {
         check_cuda(launch_c2r_fused(dtype, logn - 1, wmode, in, out, batch, idist, odist, tw, dtw, st, scale),
                    "launch fused C2R");

@@ -23,6 +23,7 @@ struct C2CCore {
     int dtype = 0, logn = 0;
     int algo = 0;  // 1 fused, 2 four-step tile launches, 3 persistent four-step, 5 three passes
     const void *tw = nullptr;
+    const void *tw_tma = nullptr;  // algo 1, fp32 2^12 .. 2^14: the persistent kernel's (fused_tma.cu)
     // persistent four-step: kernel, ring of `fs_slots` transforms, counters
     const FourStepKernel *fs = nullptr;
     // algo 5: three passes of short tiles (threepass.cu) through `ws`
@@ -51,7 +52,7 @@ struct C2CCore {
     int launches(long long batch) const;
     // strides in complex elements; four-step needs unit element strides
     void run(int inverse, const void *in, void *out, long long batch, long long idist, long long odist,
-             long long istride, long long ostride, cudaStream_t st, double scale = 1.0) const;
+             long long istride, long long ostride, cudaStream_t st, double scale = 1.0, bool host = false) const;
     // persistent four-step: the launches over `batch` transforms (dtw: the
     // DIT twiddles in real-input mode); false, with nothing launched, when
     // the input cannot be read by tensor copies (not 16-byte aligned)
@@ -122,7 +123,7 @@ struct R2CCore {
     // row pass with the DIT fused, 4 one persistent four-step launch whose
     // row items apply the DIT (3 and 4: half spectrum; other modes as 2)
     int algo = 0;
-    const void *tw = nullptr, *dtw = nullptr;
+    const void *tw = nullptr, *dtw = nullptr, *tw_tma = nullptr;
     const RowDitKernel *rowdit = nullptr;
     const void *tw_rowdit = nullptr;
     C2CCore c2c;
@@ -142,7 +143,7 @@ struct C2RCore {
     // pass that forms Z' + row pass (real_pipe.cu; the folded full spectrum
     // as 2)
     int algo = 0;
-    const void *tw = nullptr, *dtw = nullptr;
+    const void *tw = nullptr, *dtw = nullptr, *tw_tma = nullptr;
     // algo 1 whose folded full-spectrum input (2 n/2 bins) does not fit the
     // fused kernel's shared memory: that mode takes the algo 2 route
     bool fold_split = false;
