@@ -36,6 +36,7 @@ _PLANS: "OrderedDict[tuple, Plan]" = OrderedDict()
 _MAX_PLANS = 64
 # whether a functorch transform is active (taken to be so where torch cannot say)
 _functorch_active = getattr(torch._C, "_are_functorch_transforms_active", lambda: True)
+_tracing_state = torch._C._get_tracing_state
 
 
 def norm_scale(norm, n: int, inverse: bool) -> float:
@@ -195,12 +196,13 @@ class _C2R(torch.autograd.Function):
 
 def _plain(x) -> bool:
     """Whether the transform of x is nobody's business but its caller's: an
-    ordinary tensor outside autograd, forward-mode differentiation and the
-    function transforms (vmap, grad, ...).  Such calls skip the
-    autograd.Function around the kernel (10 us a call); every other one goes
-    through it and gets its results, or its errors."""
+    ordinary tensor outside autograd, forward-mode differentiation, the
+    function transforms (vmap, grad, ...) and torch.jit.trace, whose graph
+    records an autograd.Function but not the kernel inside it.  Such calls
+    skip the autograd.Function around the kernel (10 us a call); every other
+    one goes through it and gets its results, or its errors."""
     return (type(x) is torch.Tensor and not (x.requires_grad and torch.is_grad_enabled())
-            and _forward_ad._current_level < 0 and not _functorch_active())
+            and _forward_ad._current_level < 0 and not _functorch_active() and _tracing_state() is None)
 
 
 def _last(x, d: int):

@@ -63,6 +63,21 @@ def test_transforms_and_dual_tensors_take_the_general_way(gfft):
     assert GT._plain(x)
 
 
+@pytest.mark.parametrize("name", ["fft", "ifft", "rfft", "irfft", "fft2", "ifft2"])
+def test_traced_calls_run_again(gfft, name):
+    import torch
+    from genfft_gb300 import torchfft as GT
+    f = getattr(GT, name)
+    x, y = (torch.randn(4, 64, dtype=torch.float32 if name == "rfft" else torch.complex64, device="cuda")
+            for _ in range(2))
+    if name == "irfft":
+        x, y = x[:, :33].contiguous(), y[:, :33].contiguous()
+    # (a length read off a traced shape is a tensor, which irfft refuses)
+    kw = {"n": 64} if name == "irfft" else {}
+    traced = torch.jit.trace(lambda v: f(v, norm="ortho", **kw), x, check_trace=False)
+    assert torch.equal(traced(y), f(y, norm="ortho", **kw))
+
+
 def test_kept_plans_from_two_threads(gfft):
     import torch
     g = torch.Generator(device="cuda").manual_seed(3)
