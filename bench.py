@@ -600,7 +600,7 @@ def run_ragged(args):
             "config": {"workload": args.workload, "transforms": len(sizes), "sizes": "2^k, k ~ U{6..18}, seed 20240",
                        "elements": plan.elements, "step": "forward+inverse",
                        "l2": f"{bytes_exec // 2 >> 20} MB input per exec > 129 MB L2; no flush",
-                       "launch": "one persistent kernel per exec, CUDA-graph replay",
+                       "launch": f"{plan.launches} kernels per exec, CUDA-graph replay",
                        "parallelism": f"replicas x{world}"},
             "uniform_size_classes": {"gbs": round(uni_gbs, 2), "ms_per_exec": round(uni_ms, 4),
                                      "ragged_over_uniform_time_per_byte": round(exec_ms / uni_ms, 3)},
@@ -610,12 +610,13 @@ def run_ragged(args):
                          "traffic": traffic_from_profile(args.workload),
                          "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)" if peak_src == "measured"
                          else "fallback 6800 GB/s",
-                         "kernel": "k_ragged", "launches_per_exec": 1, "avg_exec_ms": round(exec_ms, 5),
+                         "kernel": "k_colpass_tma, k_rowpass_tma, k_ragged" if plan.launches > 1 else "k_ragged",
+                         "launches_per_exec": plan.launches, "avg_exec_ms": round(exec_ms, 5),
                          "algorithmic_bytes_per_exec": bytes_exec},
             "e2e": {"value": round(e2e_gbs, 2), "unit": "GB/s", "h2d_bytes_per_step": 2 * 8 * plan.elements,
                     "d2h_bytes_per_step": 2 * 8 * plan.elements, "api": "pinned copies + gfft_ragged_exec",
                     "steps": e2e_steps},
-            "gpu_launches": 2 * K, "check": max(errs), "clocks": clk.summary(),
+            "gpu_launches": 2 * K * plan.launches, "check": max(errs), "clocks": clk.summary(),
         }
         if not args.no_cpu and world == 1:
             cb, _, _ = time_cpu("ragged", "f32", 0, 0, len(sizes), budget_s=args.cpu_budget, max_reps=5)

@@ -89,6 +89,7 @@ SIGNATURES = {
     "gfft_ragged_exec_adjoint": [_P, _I, _P, _P, _P],
     "gfft_ragged_autotune": [_P, _P, _P, _P, ctypes.POINTER(_I), ctypes.POINTER(ctypes.c_double)],
     "gfft_ragged_elements": [_P, ctypes.POINTER(_LL)],
+    "gfft_ragged_launches": [_P, ctypes.POINTER(_I)],
     "gfft_status_string": [_I],
     "gfft_last_error": [],
     "gfft_version": [],
@@ -425,7 +426,7 @@ def rfft2_2x(a, b):
 
 class RaggedPlan:
     """Ragged batch of fp32 C2C transforms (sizes powers of two, 1..2^18)
-    packed back to back; one persistent graph-captured launch per exec."""
+    packed back to back; one graph launch per exec (`launches` kernels)."""
 
     def __init__(self, sizes):
         self.sizes = [int(s) for s in sizes]
@@ -436,6 +437,9 @@ class RaggedPlan:
         n = _LL()
         _check(lib().gfft_ragged_elements(self._h, ctypes.byref(n)))
         self.elements = n.value
+        k = _I()
+        _check(lib().gfft_ragged_launches(self._h, ctypes.byref(k)))
+        self.launches = k.value
         offs, pos = [], 0
         for s in self.sizes:
             offs.append(pos)

@@ -1021,6 +1021,13 @@ gfft_status gfft_ragged_elements(gfft_ragged plan, long long *elements)
         *elements = ragged_total(reinterpret_cast<RaggedPlan *>(plan));
     });
 }
+gfft_status gfft_ragged_launches(gfft_ragged plan, int *launches)
+{
+    GFFT_GUARD({
+        if (!plan || !launches) fail(GFFT_ERR_INVALID_VALUE, "NULL argument");
+        *launches = ragged_launches(reinterpret_cast<RaggedPlan *>(plan));
+    });
+}
 
 gfft_status gfft_device_error(int *code)
 {

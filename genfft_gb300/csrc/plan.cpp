@@ -67,7 +67,7 @@ static void wn_tables(int dtype, int logn, int *lo_bits, const void **lo, const 
 // the inter-pass twiddle tables of a tiles_pipe.cuh kernel over N = 2^logn,
 // E points a thread, G threads a column:
 // t1[f][t] = W_N^(f t), t < G, and t2[f][q] = W_N^(G f q), q < E, for f < N / (E G)
-static void t12_tables(int dtype, int logn, const TileKernel *k, const void **t1, const void **t2)
+void t12_tables(int dtype, int logn, const TileKernel *k, const void **t1, const void **t2)
 {
     const long long N = 1LL << logn, e = k->e, g = k->g, F = N / (e * g);
     auto fill = [N, F](long long width, long long mul) {
@@ -82,7 +82,7 @@ static void t12_tables(int dtype, int logn, const TileKernel *k, const void **t1
     *t2 = cached_table(key + "/2", dtype, F * e, fill(e, g));
 }
 
-static const void *tile_table(int dtype, const TileKernel *k, int logl, int c)
+const void *tile_table(int dtype, const TileKernel *k, int logl, int c)
 {
     return cached_table("tile/" + std::to_string(dtype) + "/" + std::to_string(logl) + "/" + std::to_string(c) +
                             "/" + std::to_string(k->threads),

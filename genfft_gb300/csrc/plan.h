@@ -228,10 +228,28 @@ cudaError_t launch_rows_bitrev(int dtype, const void *in, void *out, int logh, l
 cudaError_t launch_herm_fill(int dtype, void *out, long long H, long long W, long long ld, long long batch,
                              long long odist, cudaStream_t st);
 
+// tables of a tile kernel (plan.cpp): the Stockham twiddles of its length,
+// and the inter-pass ones of a tiles_pipe.cuh column pass over 2^logn points
+const void *tile_table(int dtype, const TileKernel *k, int logl, int c);
+void t12_tables(int dtype, int logn, const TileKernel *k, const void **t1, const void **t2);
+
 // ---- ragged batches (ragged.cu) ------------------------------------------
+// the transforms of one long size among them, on pipelined column and row
+// passes (ragged_pipe.cu): transform b of `count` starts at element off[b]
+constexpr int RAGGED_PIPE_MIN = 16, RAGGED_PIPE_MAX = 18, RAGGED_PIPE_C = 16;
+struct RaggedPipeTables {
+    const void *col = nullptr, *row = nullptr, *t1 = nullptr, *t2 = nullptr;
+};
+RaggedPipeTables ragged_pipe_tables(int logn);
+// input (16-byte aligned, `total` elements in all) to ws (transforms back to back)
+cudaError_t launch_ragged_col(int logn, int inverse, const void *in, long long total, void *ws, const long long *off,
+                              long long count, const RaggedPipeTables &tb, cudaStream_t st);
+cudaError_t launch_ragged_row(int logn, int inverse, const void *ws, void *out, const long long *off, long long count,
+                              const RaggedPipeTables &tb, cudaStream_t st);
 struct RaggedPlan;
 RaggedPlan *ragged_create(int dtype, const long long *sizes, long long count);
 void ragged_destroy(RaggedPlan *p);
+int ragged_launches(const RaggedPlan *p);
 long long ragged_total(const RaggedPlan *p);
 void ragged_exec(RaggedPlan &p, int inverse, void *out, const void *in, cudaStream_t st, bool use_graph);
 double ragged_autotune(RaggedPlan &p, void *out, const void *in, cudaStream_t st, int *best);

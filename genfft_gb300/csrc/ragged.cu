@@ -1,5 +1,5 @@
-// ragged.cu -- one persistent launch for a batch of transforms of uneven
-// power-of-two sizes (fp32, n = 2^0 .. 2^18), packed back to back.
+// ragged.cu -- a batch of transforms of uneven power-of-two sizes (fp32,
+// n = 2^0 .. 2^18), packed back to back, in one persistent launch.
 //
 // The reference transforms one size per FFT<T> object (fft.h:56-113); a
 // ragged batch there is a host loop over per-size plans.  Here a single
@@ -21,6 +21,10 @@
 // they rarely wait, and the scratch a ROW tile has read is dropped from L2
 // without a write-back.  Batches whose packing is not 16-byte aligned (sizes
 // of one point) load tiles with the compute threads instead of TMA.
+//
+// Sizes of 2^16 .. 2^18 with enough transforms take column and row passes of
+// their own before this kernel (ragged_pipe.cu; the batch's other sizes are
+// the list `rest`), where the input can be read by tensor copies.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -425,6 +429,27 @@ __global__ void __launch_bounds__(THREADS, 2) k_ragged(const Args A)
 
 using rg::Item;
 
+// the transforms of one size that go through ragged_pipe.cu
+struct RaggedClass {
+    int logn;
+    long long first, count;  // their starts: dev_class_off[first ...]
+    long long ws;            // scratch offset of the first; the others follow
+    RaggedPipeTables tables;
+};
+
+// A work list on the device.  `all` holds every transform (input off 16-byte
+// boundaries), `rest` those of no class.
+struct RaggedItems {
+    void *items = nullptr, *perm = nullptr;
+    int n = 0;
+    void release()
+    {
+        if (items) cudaFree(items);
+        if (perm) cudaFree(perm);
+        items = perm = nullptr;
+    }
+};
+
 struct RaggedPlan {
     int device = 0;
     long long count = 0, total = 0;  // transforms, elements
@@ -436,13 +461,15 @@ struct RaggedPlan {
     int large_first = 1;      // order large transforms before small ones
     int tma = 1;              // packing 16-byte aligned (no one-point transforms)
     // device state
-    void *dev_items = nullptr, *dev_perm = nullptr, *dev_off = nullptr, *dev_wsoff = nullptr;
+    RaggedItems all, rest;
+    std::vector<RaggedClass> classes;
+    void *dev_class_off = nullptr;
+    void *dev_off = nullptr, *dev_wsoff = nullptr;
     int *dev_counters = nullptr;  // [0] item counter, [1] abort, [2..count+1] col_done
     void *ws = nullptr;
     size_t ws_bytes = 0;
     const void *tw = nullptr;
     rg::Tables tab{};
-    int nitems = 0;
     int grid = 0;
     // captured graphs, keyed by (in, out, inverse)
     std::map<std::tuple<const void *, void *, int>, cudaGraphExec_t> graphs;
@@ -456,7 +483,30 @@ static void ragged_free_graphs(RaggedPlan &p)
     p.graphs.clear();
 }
 
-// (re)build the device work list for the current tuning parameters
+// Whether the `count` transforms of 2^logn points go through the pipelined
+// passes.  Those are launches of their own, column pass and row pass, before
+// the persistent kernel that takes the other sizes, so they have to fill the
+// chip by themselves: RAGGED_PIPE_POINTS points.  GB300, us an exec of 2^22 /
+// 2^23 / 2^24 points of one size beside 64 transforms of 2^12: 2^16
+// persistent 33 / 69 / 118, passes 39 / 60 / 109; 2^17 37 / 73 / 126, 42 / 62 /
+// 111; 2^18 41 / 79 / 137, 45 / 65 / 112.
+constexpr long long RAGGED_PIPE_POINTS = 1LL << 23;
+static bool ragged_pipe_takes(int logn, long long count)
+{
+    return logn >= RAGGED_PIPE_MIN && logn <= RAGGED_PIPE_MAX && (count << logn) >= RAGGED_PIPE_POINTS &&
+           count < (1LL << 24);
+}
+
+static bool in_class(const RaggedPlan &p, int logn)
+{
+    for (const RaggedClass &c : p.classes)
+        if (c.logn == logn) return true;
+    return false;
+}
+
+static void ragged_build_list(RaggedPlan &p, RaggedItems &list, bool with_classes);
+
+// (re)build the device work lists for the current tuning parameters
 static void ragged_build_items(RaggedPlan &p)
 {
     // persistent grid first: the ROW lag is measured in items in flight
@@ -467,6 +517,13 @@ static void ragged_build_items(RaggedPlan &p)
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device);
     p.grid = std::max(1, per_sm) * sms;
+    ragged_build_list(p, p.all, true);
+    if (!p.classes.empty()) ragged_build_list(p, p.rest, false);
+    ragged_free_graphs(p);
+}
+
+static void ragged_build_list(RaggedPlan &p, RaggedItems &list, bool with_classes)
+{
     const long long lag = (long long)p.grid * (rg::NS + 1) * std::max(1, p.lag_factor);
 
     std::vector<Item> items;
@@ -475,7 +532,7 @@ static void ragged_build_items(RaggedPlan &p)
     // items after the last COL tile of its transform
     std::vector<int> large;
     for (long long i = 0; i < p.count; i++)
-        if (p.logn[i] > rg::MAX_SMALL_LOGN) large.push_back((int)i);
+        if (p.logn[i] > rg::MAX_SMALL_LOGN && (with_classes || !in_class(p, p.logn[i]))) large.push_back((int)i);
     std::stable_sort(large.begin(), large.end(), [&](int x, int y) { return p.logn[x] > p.logn[y]; });
     auto cols = [&](int i) {
         const int l = p.logn[i], la = rg::split_a(l);
@@ -521,16 +578,16 @@ static void ragged_build_items(RaggedPlan &p)
         items.insert(items.end(), big.begin(), big.end());
     }
     if (perm.empty()) perm.push_back(0);
-    if (items.empty()) fail(GFFT_ERR_INVALID_SIZE, "empty ragged batch");
-    if (p.dev_items) cudaFree(p.dev_items);
-    if (p.dev_perm) cudaFree(p.dev_perm);
-    p.dev_items = p.dev_perm = nullptr;
-    check_cuda(cudaMalloc(&p.dev_items, items.size() * sizeof(Item)), "cudaMalloc(items)");
-    check_cuda(cudaMalloc(&p.dev_perm, perm.size() * sizeof(int)), "cudaMalloc(perm)");
-    check_cuda(cudaMemcpy(p.dev_items, items.data(), items.size() * sizeof(Item), cudaMemcpyHostToDevice), "items");
-    check_cuda(cudaMemcpy(p.dev_perm, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice), "perm");
-    p.nitems = (int)items.size();
-    ragged_free_graphs(p);
+    list.release();
+    list.n = (int)items.size();
+    if (items.empty()) {
+        if (with_classes) fail(GFFT_ERR_INVALID_SIZE, "empty ragged batch");
+        return;
+    }
+    check_cuda(cudaMalloc(&list.items, items.size() * sizeof(Item)), "cudaMalloc(items)");
+    check_cuda(cudaMalloc(&list.perm, perm.size() * sizeof(int)), "cudaMalloc(perm)");
+    check_cuda(cudaMemcpy(list.items, items.data(), items.size() * sizeof(Item), cudaMemcpyHostToDevice), "items");
+    check_cuda(cudaMemcpy(list.perm, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice), "perm");
 }
 
 RaggedPlan *ragged_create(int dtype, const long long *sizes, long long count)
@@ -544,18 +601,36 @@ RaggedPlan *ragged_create(int dtype, const long long *sizes, long long count)
     p->off.resize(count);
     std::vector<long long> wsoff(count, 0);
     long long pos = 0, wpos = 0;
+    long long of_size[rg::MAX_LOGN + 1] = {};
+    bool aligned[rg::MAX_LOGN + 1];  // every transform of the size starts on a multiple of RAGGED_PIPE_C
+    std::fill(std::begin(aligned), std::end(aligned), true);
     for (long long i = 0; i < count; i++) {
         if (!is_pow2(sizes[i]) || sizes[i] > (1LL << rg::MAX_LOGN))
             fail(GFFT_ERR_INVALID_SIZE, "ragged sizes must be powers of two in [1, 2^18]");
         p->logn[i] = ilog2ll(sizes[i]);
         p->off[i] = pos;
+        of_size[p->logn[i]]++;
+        if (pos % RAGGED_PIPE_C) aligned[p->logn[i]] = false;
         pos += sizes[i];
-        if (p->logn[i] > rg::MAX_SMALL_LOGN) {
+    }
+    p->total = pos;
+    // scratch: the classes' transforms back to back, then the others
+    std::vector<long long> class_off;
+    for (int l = RAGGED_PIPE_MAX; l >= RAGGED_PIPE_MIN; l--) {
+        if (!aligned[l] || !ragged_pipe_takes(l, of_size[l])) continue;
+        p->classes.push_back({l, (long long)class_off.size(), of_size[l], wpos, ragged_pipe_tables(l)});
+        for (long long i = 0; i < count; i++)
+            if (p->logn[i] == l) {
+                class_off.push_back(p->off[i]);
+                wsoff[i] = wpos;
+                wpos += sizes[i];
+            }
+    }
+    for (long long i = 0; i < count; i++)
+        if (p->logn[i] > rg::MAX_SMALL_LOGN && !in_class(*p, p->logn[i])) {
             wsoff[i] = wpos;
             wpos += sizes[i];
         }
-    }
-    p->total = pos;
     // twiddles: Stockham tables for every small length and tile length,
     // four-step split tables for every large length
     std::vector<cpx<float>> host;
@@ -583,6 +658,12 @@ RaggedPlan *ragged_create(int dtype, const long long *sizes, long long count)
     check_cuda(cudaMemcpy(p->dev_off, p->off.data(), count * sizeof(long long), cudaMemcpyHostToDevice), "off");
     check_cuda(cudaMalloc(&p->dev_wsoff, count * sizeof(long long)), "cudaMalloc(wsoff)");
     check_cuda(cudaMemcpy(p->dev_wsoff, wsoff.data(), count * sizeof(long long), cudaMemcpyHostToDevice), "wsoff");
+    if (!class_off.empty()) {
+        check_cuda(cudaMalloc(&p->dev_class_off, class_off.size() * sizeof(long long)), "cudaMalloc(class_off)");
+        check_cuda(cudaMemcpy(p->dev_class_off, class_off.data(), class_off.size() * sizeof(long long),
+                              cudaMemcpyHostToDevice),
+                   "class_off");
+    }
     check_cuda(cudaMalloc(&p->dev_counters, (count + 2) * sizeof(int)), "cudaMalloc(counters)");
     p->ws_bytes = (size_t)std::max<long long>(wpos, 1) * sizeof(cpx<float>);
     check_cuda(cudaMalloc(&p->ws, p->ws_bytes), "cudaMalloc(ragged scratch)");
@@ -606,12 +687,20 @@ void ragged_destroy(RaggedPlan *p)
     if (!p) return;
     ragged_free_graphs(*p);
     for (auto &kv : p->maps) cudaFree(kv.second);
-    for (void *q : {p->dev_items, p->dev_perm, p->dev_off, p->dev_wsoff, (void *)p->dev_counters, p->ws})
+    p->all.release();
+    p->rest.release();
+    for (void *q : {p->dev_class_off, p->dev_off, p->dev_wsoff, (void *)p->dev_counters, p->ws})
         if (q) cudaFree(q);
     delete p;
 }
 
 long long ragged_total(const RaggedPlan *p) { return p->total; }
+
+// kernels of an exec on 16-byte aligned input
+int ragged_launches(const RaggedPlan *p)
+{
+    return 2 * (int)p->classes.size() + (p->classes.empty() || p->rest.n ? 1 : 0);
+}
 
 // Tensor maps of the large transforms for input `in` (built once per
 // pointer, before any capture; nullptr when the batch cannot use TMA)
@@ -629,7 +718,7 @@ static const CUtensorMap *ragged_maps(RaggedPlan &p, const void *in, bool build)
     std::memset(h.data(), 0, h.size() * sizeof(CUtensorMap));
     for (long long t = 0; t < p.count; t++) {
         const int l = p.logn[t];
-        if (l <= rg::MAX_SMALL_LOGN) continue;
+        if (l <= rg::MAX_SMALL_LOGN || in_class(p, l)) continue;
         const int la = rg::split_a(l);
         const unsigned long long A = 1ULL << la, B = 1ULL << (l - la);
         const char *base = static_cast<const char *>(in) + (size_t)p.off[t] * sizeof(cpx<float>);
@@ -646,22 +735,34 @@ static const CUtensorMap *ragged_maps(RaggedPlan &p, const void *in, bool build)
 
 static void ragged_enqueue(RaggedPlan &p, int inverse, void *out, const void *in, cudaStream_t st)
 {
+    const bool tma = p.tma && (uintptr_t)in % 16 == 0;
+    const RaggedItems &list = tma && !p.classes.empty() ? p.rest : p.all;
+    if (tma)
+        for (const RaggedClass &c : p.classes) {
+            cpx<float> *ws = static_cast<cpx<float> *>(p.ws) + c.ws;
+            const long long *off = static_cast<const long long *>(p.dev_class_off) + c.first;
+            check_cuda(launch_ragged_col(c.logn, inverse, in, p.total, ws, off, c.count, c.tables, st),
+                       "launch ragged column pass");
+            check_cuda(launch_ragged_row(c.logn, inverse, ws, out, off, c.count, c.tables, st),
+                       "launch ragged row pass");
+        }
+    if (!list.n) return;
     check_cuda(cudaMemsetAsync(p.dev_counters, 0, (p.count + 2) * sizeof(int), st), "reset counters");
     rg::Args a;
     a.in = static_cast<const cpx<float> *>(in);
     a.out = static_cast<cpx<float> *>(out);
     a.ws = static_cast<cpx<float> *>(p.ws);
-    a.items = static_cast<const Item *>(p.dev_items);
-    a.perm = static_cast<const int *>(p.dev_perm);
+    a.items = static_cast<const Item *>(list.items);
+    a.perm = static_cast<const int *>(list.perm);
     a.off = static_cast<const long long *>(p.dev_off);
     a.wsoff = static_cast<const long long *>(p.dev_wsoff);
     a.counter = p.dev_counters;
     a.col_done = p.dev_counters + 2;
-    a.tma = p.tma && ((uintptr_t)in % 16 == 0) ? 1 : 0;
+    a.tma = tma ? 1 : 0;
     a.maps = a.tma ? ragged_maps(p, in, false) : nullptr;
     a.err = device_error_word();
     a.tw = static_cast<const cpx<float> *>(p.tw);
-    a.nitems = p.nitems;
+    a.nitems = list.n;
     a.tab = p.tab;
     void *args[] = {&a};
     const void *fn = inverse ? (const void *)rg::k_ragged<true> : (const void *)rg::k_ragged<false>;

@@ -245,10 +245,12 @@ cudaError_t launch_colpass(const TileKernel &k, int inverse, long long tiles, lo
             if (e != cudaSuccess) return e;
             unsigned *err = device_error_word();
             const long long grid = persistent_grid(fn, k.tma_threads, k.tma_smem, tiles * nbatch);
-            // (the last one: k_colpass_tma's second tensor map, unused here)
+            // (the last two: k_colpass_tma's second tensor map and the starts
+            // of packed transforms, unused here)
+            const long long *off = nullptr;
             void *args[] = {(void *)&map, (void *)&out, (void *)&ncols, (void *)&ld_out, (void *)&odist,
                             (void *)&nbatch, (void *)&tw, (void *)&tw_lo, (void *)&tw_hi, (void *)&lo_bits,
-                            (void *)&nmask, (void *)&err, scale_p, (void *)&map};
+                            (void *)&nmask, (void *)&err, scale_p, (void *)&map, (void *)&off};
             return launch_pdl(fn, dim3((unsigned)grid), dim3(k.tma_threads), args, k.tma_smem, st);
         }
     }
@@ -276,10 +278,11 @@ cudaError_t launch_colpass(const TileKernel &k, int inverse, long long tiles, lo
             cudaError_t e = ensure_smem(fn, k.tmau_smem);
             if (e != cudaSuccess) return e;
             unsigned *err = device_error_word();
+            const long long *off = nullptr;
             const long long grid = persistent_grid(fn, k.tma_threads, k.tmau_smem, tiles * nbatch);
             void *args[] = {(void *)&map[0], (void *)&out, (void *)&ncols, (void *)&ld_out, (void *)&odist,
                             (void *)&nbatch, (void *)&tw, (void *)&tw_lo, (void *)&tw_hi, (void *)&skew,
-                            (void *)&nmask, (void *)&err, scale_p, (void *)&map[1]};
+                            (void *)&nmask, (void *)&err, scale_p, (void *)&map[1], (void *)&off};
             return launch_pdl(fn, dim3((unsigned)grid), dim3(k.tma_threads), args, k.tmau_smem, st);
         }
     }
@@ -316,9 +319,10 @@ cudaError_t launch_rowpass(const TileKernel &k, int inverse, long long tiles, lo
         unsigned *err = device_error_word();
         const long long grid = persistent_grid(fn, k.tma_threads, k.tma_smem, tiles * nbatch);
         unsigned late_u = late;
+        const long long *off = nullptr;
         void *args[] = {(void *)&in,    (void *)&out,   (void *)&nrows, (void *)&ld_in, (void *)&ostride,
                         (void *)&idist, (void *)&odist, (void *)&nbatch, (void *)&tw, (void *)&err, scale_p,
-                        (void *)&late_u};
+                        (void *)&late_u, (void *)&off};
         return launch_pdl(fn, dim3((unsigned)grid), dim3(k.tma_threads), args, k.tma_smem, st);
     }
     const void *fn = inverse ? k.inv : k.fwd;

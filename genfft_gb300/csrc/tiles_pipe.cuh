@@ -203,15 +203,19 @@ namespace pipe {
 // granule wider than the tile.  (GB300, us: 5001 columns of 2^10 points 21.3
 // against 29.5 for 16-point tiles of plain loads, of 2^11 51.8 / 69.3; an
 // even count takes 16.6 and 38.4.)
-template <typename T, int LOGL, int C, int E_, int NG, int NB, bool INV, int TWM, bool U = false>
+// AT: transform b starts at element off[b] of the packed input, a multiple of
+// C, which the tensor map views as rows of ncols elements (a power of two); a
+// tile then lies in rows that start off[b] / ncols down and never straddles
+// two of them.
+template <typename T, int LOGL, int C, int E_, int NG, int NB, bool INV, int TWM, bool U = false, bool AT = false>
 __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU : LAND_COL>::THREADS, 1)
     k_colpass_tma(const __grid_constant__ CUtensorMap map, cpx<T> *__restrict__ out, long long ncols, long long ld_out,
               long long odist, long long nbatch, const cpx<T> *__restrict__ tw, const cpx<T> *__restrict__ t1,
               const cpx<T> *__restrict__ t2, int skew, unsigned late, unsigned *err, T scale,
-              const __grid_constant__ CUtensorMap map1)
+              const __grid_constant__ CUtensorMap map1, const long long *__restrict__ off = nullptr)
 {
     using Cfg = PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU : LAND_COL>;
-    static_assert(!U || TWM == 0, "plain columns");
+    static_assert(!U || (TWM == 0 && !AT), "plain columns");
     using SP = typename Cfg::SP;
     static_assert(sizeof(cpx<T>) == 8 && (TWM == 0 || TWM == 3 || TWM == 4), "fp32; no twiddle, or from t1 / t2");
     constexpr int E = SP::E, G = SP::G, N = SP::N, GT = Cfg::GT;
@@ -240,6 +244,12 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU 
     pdl_enter();  // launched by launch_pdl: waits for the previous kernel
     __syncthreads();
 
+    // AT: the start of tile i's transform, read ahead of its copy
+    auto start_of = [&](int i) {
+        const int w = w0 + i * step;
+        return w < total ? __ldg(off + (unsigned)w / (unsigned)tiles) : 0LL;
+    };
+    long long next_off = 0;
     auto issue = [&](int i) {
         const int w = w0 + i * step;
         if (w >= total) return;
@@ -254,6 +264,10 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU 
                 tensor_load_3d(S + r * Cfg::BW, &map, c0, r, b, &full[buf]);
                 tensor_load_3d(S + (N / 2 + r) * Cfg::BW, &map1, c0, r, b, &full[buf]);
             }
+        } else if constexpr (AT) {
+            const long long at = (i < NB ? start_of(i) : next_off) + c0;
+            const int y = (int)(at / ncols), x = (int)(at & (ncols - 1));
+            for (int r = 0; r < N; r += Cfg::BOXR) tensor_load_3d(S + r * C, &map, x, y + r, 0, &full[buf]);
         } else {
             for (int r = 0; r < N; r += Cfg::BOXR) tensor_load_3d(S + r * C, &map, c0, r, b, &full[buf]);
         }
@@ -267,6 +281,7 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU 
         // the tile's t2 values go to the group's two buffers in turn: slower warps of
         // the group may still read the other one for the tile before
         cpx<T> *const t2s = t2b + (i / NG & 1) * Cfg::T2;
+        if constexpr (AT) next_off = start_of(i + NB);
         cpx<T> w1{(T)0, (T)0};
         if constexpr (TWM != 0) {
             const unsigned f = TWM == 3 ? (unsigned)(active ? col : 0) : (unsigned)b;
@@ -318,12 +333,13 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU 
 
 // Row pass with transposed store: see k_rowpass (tiles.cuh).  The rows land
 // RP apart and thread (s, t) holds points of row s, s fastest, so the
-// outputs leave the registers in runs of C without a transpose.
-template <typename T, int LOGL, int C, int E_, int NG, int NB, bool INV>
+// outputs leave the registers in runs of C without a transpose.  AT: the
+// output of transform b starts at element off[b].
+template <typename T, int LOGL, int C, int E_, int NG, int NB, bool INV, bool AT = false>
 __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, LAND_ROW>::THREADS, 1)
     k_rowpass_tma(const cpx<T> *__restrict__ in, cpx<T> *__restrict__ out, long long nrows, long long ld_in,
               long long ostride, long long idist, long long odist, long long nbatch, const cpx<T> *__restrict__ tw,
-              unsigned *err, T scale, unsigned late)
+              unsigned *err, T scale, unsigned late, const long long *__restrict__ off = nullptr)
 {
     using Cfg = PipeCfg<T, LOGL, C, E_, NG, NB, LAND_ROW>;
     using SP = typename Cfg::SP;
@@ -370,6 +386,9 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, LAND_ROW>::THR
         cpx<T> *const S = stage0 + (size_t)buf * Cfg::STAGE;
         const int wb = (int)((unsigned)w / (unsigned)tiles);
         const long long b = wb, row = (long long)(w - wb * tiles) * C + s;
+        long long start;
+        if constexpr (AT) start = __ldg(off + b);
+        else start = b * odist;
         const bool ok = stage_wait(&full[buf], &seq[buf], i, par);
         cpx<T> v[E];
 #pragma unroll
@@ -385,7 +404,7 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, LAND_ROW>::THR
             [&]() { landed = bar_group_and(bar, GT, ok); });
         if (!landed) return false;
         if (row < nrows) {
-            cpx<T> *dst = out + b * odist + row + (long long)t * ostride;
+            cpx<T> *dst = out + start + row + (long long)t * ostride;
             const long long st = (long long)G * ostride;
 #pragma unroll
             for (int q = 0; q < E; q++, dst += st) stcs_c(dst, scl(v[q], scale));

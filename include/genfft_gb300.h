@@ -238,6 +238,8 @@ gfft_status gfft_ragged_autotune(gfft_ragged plan, void *out, const void *in, vo
                                  double *ms);
 /* total complex elements of the packed batch */
 gfft_status gfft_ragged_elements(gfft_ragged plan, long long *elements);
+/* kernels one exec launches on 16-byte aligned input */
+gfft_status gfft_ragged_launches(gfft_ragged plan, int *launches);
 
 /* Device-side error status of this device's kernels since the last call
  * (synchronous): *code = 0 and GFFT_OK if none; otherwise the recorded
