@@ -63,6 +63,7 @@ SIGNATURES = {
     "gfft_exec": [_P, _I, _P, _P, _P],
     "gfft_exec_host": [_P, _I, _P, _P],
     "gfft_exec_adjoint": [_P, _I, _P, _P, _P],
+    "gfft_exec_adjoint_scaled": [_P, _I, ctypes.c_double, _P, _P, _P],
     "gfft_exec_scaled": [_P, _I, ctypes.c_double, _P, _P, _P],
     "gfft_plan_launches": [_P, ctypes.POINTER(_I)],
     "gfft_plan_launches_dir": [_P, _I, ctypes.POINTER(_I)],
@@ -181,8 +182,13 @@ class Plan:
     def adjoint_ptr(self, out_ptr: int, in_ptr: int, inverse: bool = False, stream_ptr: int = 0):
         _check(lib().gfft_exec_adjoint(self._h, int(inverse), out_ptr, in_ptr, stream_ptr))
 
-    def adjoint(self, out, g, inverse: bool = False, stream=None):
-        self.adjoint_ptr(out.data_ptr(), g.data_ptr(), inverse, _stream_ptr(stream))
+    def adjoint(self, out, g, inverse: bool = False, stream=None, scale: float = 1.0):
+        """Adjoint of exec with the same `inverse` and `scale`."""
+        if scale == 1.0:
+            self.adjoint_ptr(out.data_ptr(), g.data_ptr(), inverse, _stream_ptr(stream))
+        else:
+            _check(lib().gfft_exec_adjoint_scaled(self._h, int(inverse), float(scale), out.data_ptr(), g.data_ptr(),
+                                                  _stream_ptr(stream)))
         return out
 
     def exec_host_ptr(self, out_ptr: int, in_ptr: int, inverse: bool = False):

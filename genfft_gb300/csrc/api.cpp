@@ -391,7 +391,9 @@ static void exec_plan(gfft_plan_s &p, int inverse, void *out, const void *in, co
 
 // Adjoint of the plan's transform in direction `inverse` (reverse-mode
 // differentiation: grad_in = A^H grad_out in PyTorch's convention).
-static void exec_adjoint(gfft_plan_s &p, int inverse, void *out, const void *in, const Layout &L, cudaStream_t st)
+// `scale` multiplies every output.
+static void exec_adjoint(gfft_plan_s &p, int inverse, void *out, const void *in, const Layout &L, cudaStream_t st,
+                         double scale = 1.0)
 {
     const gfft_desc &d = p.d;
     switch (d.kind) {
@@ -402,7 +404,7 @@ static void exec_adjoint(gfft_plan_s &p, int inverse, void *out, const void *in,
         // inverse) transform; the output layout becomes the input layout
         if (d.flags & GFFT_FLAG_BITREV_INPUT) fail(GFFT_ERR_UNSUPPORTED, "adjoint of a bit-reversed-input plan");
         Layout A{L.batch, L.ostride, L.odist, L.istride, L.idist};
-        exec_plan(p, !inverse, out, in, A, st);
+        exec_plan(p, !inverse, out, in, A, st, scale);
         break;
     }
     case GFFT_KIND_R2C: {
@@ -413,14 +415,14 @@ static void exec_adjoint(gfft_plan_s &p, int inverse, void *out, const void *in,
             check_ptr(in, cb, "in");
             check_ptr(out, rb, "out");
             const int w = (d.flags & GFFT_FLAG_HALF_SPECTRUM) ? 1 : 2;
-            p.c2r.run(in, out, L.batch, L.odist, L.idist, w, st);
+            p.c2r.run(in, out, L.batch, L.odist, L.idist, w, st, scale);
         } else {
             // adjoint of the half-spectrum C2R: R2C with interior bins doubled
             check_ptr(in, rb, "in");
             check_ptr(out, cb, "out");
             if (!(d.flags & GFFT_FLAG_HALF_SPECTRUM))
                 fail(GFFT_ERR_UNSUPPORTED, "adjoint of the inverse needs a half-spectrum plan");
-            p.r2c.run(in, out, L.batch, L.idist, L.odist, st, 2);
+            p.r2c.run(in, out, L.batch, L.idist, L.odist, st, 2, scale);
         }
         break;
     }
@@ -735,6 +737,15 @@ gfft_status gfft_exec_adjoint(gfft_plan plan, int inverse, void *out, const void
     GFFT_GUARD({
         gfft_plan_s *p = checked(plan);
         exec_adjoint(*p, inverse != 0, out, in, plan_layout(*p), (cudaStream_t)stream);
+    });
+}
+
+gfft_status gfft_exec_adjoint_scaled(gfft_plan plan, int inverse, double scale, void *out, const void *in,
+                                     void *stream)
+{
+    GFFT_GUARD({
+        gfft_plan_s *p = checked(plan);
+        exec_adjoint(*p, inverse != 0, out, in, plan_layout(*p), (cudaStream_t)stream, scale);
     });
 }
 

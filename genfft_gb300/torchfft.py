@@ -173,8 +173,7 @@ class _R2C(torch.autograd.Function):
         p = _plan(KIND_R2C, _code(g), n, 0, g.numel() // g.shape[-1], FLAG_HALF_SPECTRUM)
         rdt = torch.float64 if g.dtype == torch.complex128 else torch.float32
         gx = torch.empty(*g.shape[:-1], n, dtype=rdt, device=g.device)
-        p.adjoint(gx, g, False)
-        return gx.mul_(ctx.scale) if ctx.scale != 1.0 else gx, None
+        return p.adjoint(gx, g, False, scale=ctx.scale), None
 
 
 class _C2R(torch.autograd.Function):
@@ -190,8 +189,7 @@ class _C2R(torch.autograd.Function):
         p = _plan(KIND_R2C, _code(g), n, 0, g.numel() // n, FLAG_HALF_SPECTRUM)
         cdt = torch.complex128 if g.dtype == torch.float64 else torch.complex64
         gy = torch.empty(*g.shape[:-1], n // 2 + 1, dtype=cdt, device=g.device)
-        p.adjoint(gy, g, True)
-        return (gy.mul_(ctx.scale) if ctx.scale != 1.0 else gy), None, None
+        return p.adjoint(gy, g, True, scale=ctx.scale), None, None
 
 
 def _plain(x) -> bool:

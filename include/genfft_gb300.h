@@ -117,6 +117,10 @@ gfft_status gfft_exec_scaled(gfft_plan plan, int inverse, double scale, void *ou
  * full spectrum folded); C2R: an R2C with interior bins doubled.  `in` has
  * the layout of the transform's output, `out` that of its input. */
 gfft_status gfft_exec_adjoint(gfft_plan plan, int inverse, void *out, const void *in, void *stream);
+/* gfft_exec_adjoint with every output multiplied by `scale` inside the kernel
+ * that writes it: the adjoint of gfft_exec_scaled. */
+gfft_status gfft_exec_adjoint_scaled(gfft_plan plan, int inverse, double scale, void *out, const void *in,
+                                     void *stream);
 /* Same transform on HOST buffers (the reference's calling convention):
  * copies in, transforms and copies out in pipelined chunks, synchronously.
  * Pinned host memory gives full link bandwidth; pageable memory works.
