@@ -79,12 +79,15 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&r)[32])
 // even, from a 16-byte boundary; C2R: bins, from any).  Out: odist apart (R2C:
 // bins; C2R: complex elements).  interior: the factor of bins 1 .. N - 1, 2
 // for the adjoint of C2R (R2C), 1/2 for the adjoint of R2C (C2R), else 1.
-template <int LOGN, int NG, int KIND, bool INV>
+// AT (C2C): transform w is at element off[w], even, of in and out instead.
+template <int LOGN, int NG, int KIND, bool INV, bool AT = false>
 __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
     k_fused_tma(const c32 *__restrict__ in, c32 *__restrict__ out, int batch, long long idist, long long odist,
-                const c32 *__restrict__ tw, const c32 *__restrict__ dtw, unsigned *err, float scale, float interior)
+                const c32 *__restrict__ tw, const c32 *__restrict__ dtw, unsigned *err, float scale, float interior,
+                const long long *__restrict__ off)
 {
     using Cfg = FusedTmaCfg<LOGN, NG, KIND>;
+    static_assert(!AT || KIND == FUSED_C2C, "packed transforms are C2C");
     using SP = typename Cfg::SP;
     constexpr int N = Cfg::N, E = Cfg::E, G = Cfg::G, R0 = SP::R0;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -107,9 +110,13 @@ __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
     // one that still had its own to allocate would wait for ours while we wait
     // for it), and later grids may come in only once it is taken.
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    // AT: where this transform and the next one start, read ahead of the copy
+    auto start_of = [&](int w) { return w < batch ? __ldg(off + w) : 0LL; };
+    long long at = 0, next_at = 0;
+    if constexpr (AT) next_at = start_of(first);
     auto issue = [&](int w) {
         if (w >= batch) return;
-        const c32 *src = in + (long long)w * idist;
+        const c32 *src = in + (AT ? next_at : (long long)w * idist);
         if constexpr (KIND == FUSED_C2R) {
             // N + 1 bins and what shares their first and last 16 bytes
             const uintptr_t a = (uintptr_t)src & ~(uintptr_t)15, e = ((uintptr_t)(src + N + 1) + 15) & ~(uintptr_t)15;
@@ -154,6 +161,10 @@ __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
 
     uint32_t par = 0;
     for (int w = first; w < batch; w += step, par ^= 1) {
+        if constexpr (AT) {
+            at = next_at;
+            next_at = start_of(w + step);
+        }
         const bool ok = mbar_wait(full, par);
         __syncwarp();
         c32 v[E];
@@ -232,7 +243,7 @@ __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
                 if (c * 16 + j > 0) v[c * 16 + j] = twmul<INV>(v[c * 16 + j], c32{r[2 * j], r[2 * j + 1]});
         }
         dft<E, INV, float>(v);
-        c32 *const dst = out + (long long)w * odist;
+        c32 *const dst = out + (AT ? at : (long long)w * odist);
         if constexpr (KIND != FUSED_R2C) {
 #pragma unroll
             for (int q = 0; q < E; q++) stcs_c(dst + t + q * G, scl(v[q], scale));
@@ -274,15 +285,23 @@ __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
 
 namespace {
 struct Entry {
-    const void *fn[4];  // C2C forward and inverse, R2C, C2R
+    const void *fn[6];  // C2C forward and inverse, R2C, C2R, packed C2C forward and inverse
     int groups;
     size_t smem[3];     // by kind
 };
+// (packed: 2^13 and 2^14 only, see ragged.cu)
+template <int LOGN, int NG, bool INV>
+const void *packed_fn()
+{
+    if constexpr (LOGN > 12) return (const void *)&k_fused_tma<LOGN, NG, FUSED_C2C, INV, true>;
+    else return nullptr;
+}
 template <int LOGN, int NG>
 Entry make_entry()
 {
     return Entry{{(const void *)&k_fused_tma<LOGN, NG, FUSED_C2C, false>, (const void *)&k_fused_tma<LOGN, NG, FUSED_C2C, true>,
-                  (const void *)&k_fused_tma<LOGN, NG, FUSED_R2C, false>, (const void *)&k_fused_tma<LOGN, NG, FUSED_C2R, true>},
+                  (const void *)&k_fused_tma<LOGN, NG, FUSED_R2C, false>, (const void *)&k_fused_tma<LOGN, NG, FUSED_C2R, true>,
+                  packed_fn<LOGN, NG, false>(), packed_fn<LOGN, NG, true>()},
                  NG,
                  {FusedTmaCfg<LOGN, NG, FUSED_C2C>::SMEM, FusedTmaCfg<LOGN, NG, FUSED_R2C>::SMEM,
                   FusedTmaCfg<LOGN, NG, FUSED_C2R>::SMEM}};
@@ -294,7 +313,8 @@ const Entry &entry(int logn)
 }
 
 cudaError_t launch(int logn, int kind, int fn_i, const void *in, void *out, long long nbatch, long long idist,
-                   long long odist, const void *tw, const void *dtw, double sc, float interior, cudaStream_t st)
+                   long long odist, const void *tw, const void *dtw, double sc, float interior, cudaStream_t st,
+                   const long long *off = nullptr)
 {
     const Entry &e = entry(logn);
     const void *fn = e.fn[fn_i];
@@ -305,7 +325,7 @@ cudaError_t launch(int logn, int kind, int fn_i, const void *in, void *out, long
     float scale = (float)sc;
     const long long grid = std::min<long long>((nbatch + e.groups - 1) / e.groups, sm_count());
     void *args[] = {(void *)&in, (void *)&out, (void *)&batch, (void *)&idist, (void *)&odist, (void *)&tw,
-                    (void *)&dtw, (void *)&err, (void *)&scale, (void *)&interior};
+                    (void *)&dtw, (void *)&err, (void *)&scale, (void *)&interior, (void *)&off};
     return launch_pdl(fn, dim3((unsigned)grid), dim3(512), args, e.smem[kind], st);
 }
 }  // namespace
@@ -343,6 +363,11 @@ cudaError_t launch_fused_tma_c2c(int logn, int inverse, const FusedC2CArgs &a, c
 {
     return launch(logn, FUSED_C2C, inverse ? 1 : 0, a.in, a.out, a.batch, a.idist, a.odist, a.tw_tma, nullptr, a.scale,
                   1.f, st);
+}
+cudaError_t launch_fused_tma_at(int logn, int inverse, const void *in, void *out, const long long *off, long long count,
+                                const void *tw, cudaStream_t st)
+{
+    return launch(logn, FUSED_C2C, inverse ? 5 : 4, in, out, count, 0, 0, tw, nullptr, 1.0, 1.f, st, off);
 }
 cudaError_t launch_fused_tma_r2c(int logh, bool x2, const void *in, void *out, long long batch, long long idist,
                                  long long odist, const void *tw, const void *dtw, cudaStream_t st, double scale)

@@ -48,6 +48,9 @@ size_t fused_tma_twiddle_count(int logn);
 void fused_tma_twiddle_fill(int logn, void *host_buf);
 bool fused_tma_takes(int logn, bool real, long long batch);
 cudaError_t launch_fused_tma_c2c(int logn, int inverse, const FusedC2CArgs &a, cudaStream_t st);
+// C2C of packed transforms: number w is at element off[w], even
+cudaError_t launch_fused_tma_at(int logn, int inverse, const void *in, void *out, const long long *off, long long count,
+                                const void *tw, cudaStream_t st);
 // distances in complex elements; x2 / half: interior bins doubled / halved
 cudaError_t launch_fused_tma_r2c(int logh, bool x2, const void *in, void *out, long long batch, long long idist,
                                  long long odist, const void *tw, const void *dtw, cudaStream_t st, double scale);

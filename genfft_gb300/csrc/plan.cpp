@@ -90,7 +90,7 @@ const void *tile_table(int dtype, const TileKernel *k, int logl, int c)
 }
 
 // the Stockham table of the persistent fused kernels (fused_tma.cu), or null
-static const void *fused_tma_table(int dtype, int logn)
+const void *fused_tma_table(int dtype, int logn)
 {
     if (dtype != GFFT_F32 || logn < FUSED_TMA_MIN || logn > FUSED_TMA_MAX) return nullptr;
     return cached_table("fusedtma/" + std::to_string(logn), dtype, fused_tma_twiddle_count(logn),

@@ -232,6 +232,8 @@ cudaError_t launch_herm_fill(int dtype, void *out, long long H, long long W, lon
 // and the inter-pass ones of a tiles_pipe.cuh column pass over 2^logn points
 const void *tile_table(int dtype, const TileKernel *k, int logl, int c);
 void t12_tables(int dtype, int logn, const TileKernel *k, const void **t1, const void **t2);
+// that of the persistent fused kernels (fused_tma.cu), or null
+const void *fused_tma_table(int dtype, int logn);
 
 // ---- ragged batches (ragged.cu) ------------------------------------------
 // the transforms of one long size among them, on pipelined column and row
@@ -239,6 +241,7 @@ void t12_tables(int dtype, int logn, const TileKernel *k, const void **t1, const
 constexpr int RAGGED_PIPE_MIN = 16, RAGGED_PIPE_MAX = 18, RAGGED_PIPE_C = 16;
 struct RaggedPipeTables {
     const void *col = nullptr, *row = nullptr, *t1 = nullptr, *t2 = nullptr;
+    const void *fused = nullptr;  // sizes of the persistent fused kernel (fused_tma.cu) instead
 };
 RaggedPipeTables ragged_pipe_tables(int logn);
 // input (16-byte aligned, `total` elements in all) to ws (transforms back to back)

@@ -23,8 +23,9 @@
 // of one point) load tiles with the compute threads instead of TMA.
 //
 // Sizes of 2^16 .. 2^18 with enough transforms take column and row passes of
-// their own before this kernel (ragged_pipe.cu; the batch's other sizes are
-// the list `rest`), where the input can be read by tensor copies.
+// their own before this kernel (ragged_pipe.cu), those of 2^13 and 2^14 the
+// persistent fused kernel (fused_tma.cu), where the input can be read by
+// tensor copies; the batch's other sizes are the list `rest`.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -429,7 +430,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_ragged(const Args A)
 
 using rg::Item;
 
-// the transforms of one size that go through ragged_pipe.cu
+// the transforms of one size that go through ragged_pipe.cu or fused_tma.cu
 struct RaggedClass {
     int logn;
     long long first, count;  // their starts: dev_class_off[first ...]
@@ -495,6 +496,14 @@ static bool ragged_pipe_takes(int logn, long long count)
 {
     return logn >= RAGGED_PIPE_MIN && logn <= RAGGED_PIPE_MAX && (count << logn) >= RAGGED_PIPE_POINTS &&
            count < (1LL << 24);
+}
+// ... or, for 2^13 and 2^14, through the persistent fused kernel: one pass of
+// HBM traffic instead of two, a launch of its own (GB300, us an exec of 2^22 /
+// 2^23 / 2^24 points beside 64 transforms of 2^12: 2^13 persistent ragged kernel
+// 35 / 69 / 119, fused 32 / 44 / 70; 2^14 34 / 67 / 119, 31 / 49 / 76).
+static bool ragged_fused_takes(int logn, long long count)
+{
+    return (logn == 13 || logn == 14) && (count << logn) >= RAGGED_PIPE_POINTS && fused_tma_takes(logn, false, count);
 }
 
 static bool in_class(const RaggedPlan &p, int logn)
@@ -616,9 +625,13 @@ RaggedPlan *ragged_create(int dtype, const long long *sizes, long long count)
     p->total = pos;
     // scratch: the classes' transforms back to back, then the others
     std::vector<long long> class_off;
-    for (int l = RAGGED_PIPE_MAX; l >= RAGGED_PIPE_MIN; l--) {
-        if (!aligned[l] || !ragged_pipe_takes(l, of_size[l])) continue;
-        p->classes.push_back({l, (long long)class_off.size(), of_size[l], wpos, ragged_pipe_tables(l)});
+    for (int l = RAGGED_PIPE_MAX; l > rg::MAX_SMALL_LOGN; l--) {
+        if (!aligned[l]) continue;
+        RaggedPipeTables tables;
+        if (ragged_pipe_takes(l, of_size[l])) tables = ragged_pipe_tables(l);
+        else if (ragged_fused_takes(l, of_size[l])) tables.fused = fused_tma_table(GFFT_F32, l);
+        else continue;
+        p->classes.push_back({l, (long long)class_off.size(), of_size[l], wpos, tables});
         for (long long i = 0; i < count; i++)
             if (p->logn[i] == l) {
                 class_off.push_back(p->off[i]);
@@ -699,7 +712,9 @@ long long ragged_total(const RaggedPlan *p) { return p->total; }
 // kernels of an exec on 16-byte aligned input
 int ragged_launches(const RaggedPlan *p)
 {
-    return 2 * (int)p->classes.size() + (p->classes.empty() || p->rest.n ? 1 : 0);
+    int n = p->classes.empty() || p->rest.n ? 1 : 0;
+    for (const RaggedClass &c : p->classes) n += c.tables.fused ? 1 : 2;
+    return n;
 }
 
 // Tensor maps of the large transforms for input `in` (built once per
@@ -741,6 +756,11 @@ static void ragged_enqueue(RaggedPlan &p, int inverse, void *out, const void *in
         for (const RaggedClass &c : p.classes) {
             cpx<float> *ws = static_cast<cpx<float> *>(p.ws) + c.ws;
             const long long *off = static_cast<const long long *>(p.dev_class_off) + c.first;
+            if (c.tables.fused) {
+                check_cuda(launch_fused_tma_at(c.logn, inverse, in, out, off, c.count, c.tables.fused, st),
+                           "launch ragged fused");
+                continue;
+            }
             check_cuda(launch_ragged_col(c.logn, inverse, in, p.total, ws, off, c.count, c.tables, st),
                        "launch ragged column pass");
             check_cuda(launch_ragged_row(c.logn, inverse, ws, out, off, c.count, c.tables, st),

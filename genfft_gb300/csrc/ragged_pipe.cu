@@ -8,7 +8,7 @@
 // persistent ragged kernel (16 points a thread) take three and two.  GB300,
 // us an exec of 2^26 points of one size, persistent kernel / these passes:
 // 2^16 417 / 365, 2^17 448 / 350, 2^18 490 / 359; 10000 transforms of
-// 2^6 .. 2^18, forward and inverse, 5400 / 4210.
+// 2^6 .. 2^18, forward and inverse, 5400 / 4210 (the rest unchanged).
 #include <algorithm>
 
 #include "internal.h"

@@ -15,6 +15,9 @@ BATCHES = [  # sizes, kernels of an exec
     ([1 << 18] * (POINTS >> 18) + [1 << 17, 2], 3),         # only one size has enough
     ([1 << 17] * ((POINTS >> 17) - 1), 1),                 # one too few
     ([8] + [1 << 16] * (POINTS >> 16), 1),                  # starts off multiples of 16
+    ([16] + [1 << 14] * (POINTS >> 14) + [64] + [1 << 13] * ((POINTS >> 13) + 1), 3),  # the fused kernel
+    ([1 << 13] * (POINTS >> 13), 1),
+    ([16] + [1 << 14] * ((POINTS >> 14) - 1), 1),
     ([1] + [1 << 16] * (POINTS >> 16), 1),                  # one-point transforms: no copies at all
 ]
 
