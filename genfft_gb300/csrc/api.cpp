@@ -195,6 +195,7 @@ static gfft_plan_s *make_plan(const gfft_desc &in)
     apply_defaults(d);
     check_layout(d);
     check_device();
+    device_error_word();  // allocated now: a plan's first exec may be inside a stream capture
     std::unique_ptr<gfft_plan_s> p(new gfft_plan_s());
     check_cuda(cudaGetDevice(&p->device), "cudaGetDevice");
     p->d = d;

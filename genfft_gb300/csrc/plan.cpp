@@ -248,7 +248,6 @@ void C2CCore::init(int dtype_, int logn_, long long batch_hint, int path, bool r
         ws_bytes = (size_t)fs_slots * (size_t)N * cplx_bytes(dtype);
         check_cuda(cudaMalloc(&ws, ws_bytes), "cudaMalloc(workspace)");
         check_cuda(cudaMalloc(&fs_ctr, (size_t)(2 + 2 * fs_slots) * sizeof(int)), "cudaMalloc(counters)");
-        device_error_word();  // allocated now, never inside a stream capture
         algo = 3;
         return;
     }
