@@ -152,6 +152,29 @@ def _dtype_code(t) -> int:
     return code
 
 
+def _resolved(x, stream=None):
+    """x without a pending conjugation or negation: the kernels read the
+    values that are stored, and is_contiguous() / contiguous() say nothing
+    about either.  Made on the stream that reads it."""
+    if not (x.is_conj() or x.is_neg()):
+        return x
+    with torch.cuda.stream(stream):
+        return x.resolve_conj().resolve_neg()
+
+
+def _dense(x):
+    """x as the kernels read it: contiguous, its stored values its own."""
+    return _resolved(x).contiguous()
+
+
+def _stored(out):
+    """out, which the kernels write to (in place: read from too): refused
+    where a pending conjugation or negation would change what is there."""
+    if out.is_conj() or out.is_neg():
+        raise ValueError("an output must not be a lazily conjugated or negated view")
+    return out
+
+
 class Plan:
     """A gfft_plan (see include/genfft_gb300.h).  Sizes/strides in elements."""
 
@@ -172,6 +195,7 @@ class Plan:
     def exec(self, out, x, inverse: bool = False, stream=None, scale: float = 1.0):
         """Run on torch CUDA tensors (current stream); `scale` multiplies every
         output inside the kernel that writes it."""
+        x, _ = _resolved(x, stream), _stored(out)
         if scale == 1.0:
             self.exec_ptr(out.data_ptr(), x.data_ptr(), inverse, _stream_ptr(stream))
         else:
@@ -184,6 +208,7 @@ class Plan:
 
     def adjoint(self, out, g, inverse: bool = False, stream=None, scale: float = 1.0):
         """Adjoint of exec with the same `inverse` and `scale`."""
+        g, _ = _resolved(g, stream), _stored(out)
         if scale == 1.0:
             self.adjoint_ptr(out.data_ptr(), g.data_ptr(), inverse, _stream_ptr(stream))
         else:
@@ -257,19 +282,20 @@ def _check_cuda_tensor(x, name="x"):
         raise ValueError(f"{name} must be a CUDA tensor")
     if not x.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
+    return _resolved(x)
 
 
 def fft(x, inverse: bool = False, out=None):
     """Batched C2C over the last dimension (FFT<T>::transform<inv>, fft.h:80-85).
     The inverse is unscaled."""
-    _check_cuda_tensor(x)
+    x = _check_cuda_tensor(x)
     if x.dtype not in _COMPLEX:
         raise TypeError("fft expects complex64/complex128")
     n = x.shape[-1]
     batch = x.numel() // n if n else 0
     if out is None:
         out = torch.empty_like(x)
-    _check(lib().gfft_fft_transform(_dtype_code(x), n, batch, int(inverse), out.data_ptr(),
+    _check(lib().gfft_fft_transform(_dtype_code(x), n, batch, int(inverse), _stored(out).data_ptr(),
                                     x.data_ptr(), _stream_ptr()))
     return out
 
@@ -281,7 +307,7 @@ def fft_tc(x, inverse: bool = False, mode: int = MODE_TC_FP16, out=None):
     """Batched fp32 C2C over the last dimension (n = 256, 4096 or 65536) on
     the split-precision tensor-core path (mode MODE_TC_FP16 or MODE_TC_BF16).
     Same conventions as fft(): unscaled inverse."""
-    _check_cuda_tensor(x)
+    x = _check_cuda_tensor(x)
     if x.dtype != torch.complex64:
         raise TypeError("fft_tc expects complex64")
     n = x.shape[-1]
@@ -307,7 +333,7 @@ def _cdtype_for_real(x):
 def fft_no_scramble(x, inverse: bool = False):
     """In place on x: bit-reversed input order, natural output
     (FFT<T>::transform_no_scramble, fft.h:69-73)."""
-    _check_cuda_tensor(x)
+    _check_cuda_tensor(_stored(x))
     n = x.shape[-1]
     _check(lib().gfft_fft_transform_no_scramble(_dtype_code(x), n, x.numel() // n, int(inverse), x.data_ptr(),
                                                 _stream_ptr()))
@@ -317,7 +343,7 @@ def fft_no_scramble(x, inverse: bool = False):
 def rfft(x, half: bool = True, out=None):
     """RealFFT<T>::forward over the last dimension (FFTReal.h:204-213):
     n reals -> n/2+1 bins (half) or the full Hermitian n bins."""
-    _check_cuda_tensor(x)
+    x = _check_cuda_tensor(x)
     if x.dtype not in _REAL:
         raise TypeError("rfft expects float32/float64")
     n = x.shape[-1]
@@ -332,7 +358,7 @@ def rfft(x, half: bool = True, out=None):
 
 def fft_real_input(x):
     """FFT<T>::transform_real (fft.h:90-94): full complex spectrum of reals."""
-    _check_cuda_tensor(x)
+    x = _check_cuda_tensor(x)
     n = x.shape[-1]
     out = torch.empty(*x.shape, dtype=_cdtype_for_real(x), device=x.device)
     _check(lib().gfft_fft_transform_real(_dtype_code(x), n, x.numel() // n, out.data_ptr(), x.data_ptr(),
@@ -342,8 +368,8 @@ def fft_real_input(x):
 
 def fft_interleave(a, b):
     """FFT<T>::transform_interleave (fft.h:100-105): FFT of a + i b (1D)."""
-    _check_cuda_tensor(a, "a")
-    _check_cuda_tensor(b, "b")
+    a = _check_cuda_tensor(a, "a")
+    b = _check_cuda_tensor(b, "b")
     n = a.shape[-1]
     out = torch.empty(n, dtype=_cdtype_for_real(a), device=a.device)
     _check(lib().gfft_fft_transform_interleave(_dtype_code(a), n, out.data_ptr(), a.data_ptr(), b.data_ptr(),
@@ -353,7 +379,7 @@ def fft_interleave(a, b):
 
 def separate_2x(z):
     """separate_2x_real_FFT (FFTReal.h:34-66) -> (X, Y)."""
-    _check_cuda_tensor(z, "z")
+    z = _check_cuda_tensor(z, "z")
     n = z.shape[-1]
     a, b = torch.empty_like(z), torch.empty_like(z)
     _check(lib().gfft_separate_2x_real_fft(_dtype_code(z), n, a.data_ptr(), b.data_ptr(), z.data_ptr(),
@@ -364,7 +390,7 @@ def separate_2x(z):
 def dit(z, n: int, half: bool):
     """DIT<T>(n).apply on an n/2-point spectrum z (fft.h:180-188); returns
     an n-element buffer (only n/2+1 written when half)."""
-    _check_cuda_tensor(z, "z")
+    z = _check_cuda_tensor(z, "z")
     out = torch.zeros(n, dtype=z.dtype, device=z.device)
     buf = torch.zeros(n, dtype=z.dtype, device=z.device)
     buf[: z.shape[-1]] = z
@@ -374,18 +400,18 @@ def dit(z, n: int, half: bool):
 
 def fft_vert(x, inverse: bool = False, out=None):
     """FFTVert<T>(rows).transform on an [rows, cols] tensor (fft.h:145-150)."""
-    _check_cuda_tensor(x)
+    x = _check_cuda_tensor(x)
     rows, cols = x.shape
     if out is None:
         out = torch.empty_like(x)
-    _check(lib().gfft_vert_transform(_dtype_code(x), rows, int(inverse), out.data_ptr(), cols, x.data_ptr(),
-                                     cols, cols, _stream_ptr()))
+    _check(lib().gfft_vert_transform(_dtype_code(x), rows, int(inverse), _stored(out).data_ptr(), cols,
+                                     x.data_ptr(), cols, cols, _stream_ptr()))
     return out
 
 
 def fft_vert_no_scramble(x, inverse: bool = False):
     """FFTVert<T>::transform_no_scramble in place (rows bit-reversed)."""
-    _check_cuda_tensor(x)
+    _check_cuda_tensor(_stored(x))
     rows, cols = x.shape
     _check(lib().gfft_vert_transform_no_scramble(_dtype_code(x), rows, int(inverse), x.data_ptr(), cols, cols,
                                                  _stream_ptr()))
@@ -395,7 +421,7 @@ def fft_vert_no_scramble(x, inverse: bool = False):
 def fft2(x, inverse: bool = False, out=None):
     """FFT2D<T>(W, H).transform on [..., H, W] (fft.h:213-218); batched over
     leading dimensions through a plan."""
-    _check_cuda_tensor(x)
+    x = _check_cuda_tensor(x)
     H, W = x.shape[-2:]
     batch = x.numel() // (H * W)
     if out is None:
@@ -408,7 +434,7 @@ def fft2(x, inverse: bool = False, out=None):
 def rfft2(x, half: bool = False, out=None):
     """RealFFT2D<T>(W, H).forward on [..., H, W] reals (FFTReal.h:83-104):
     full-width Hermitian [H, W] output, or [H, W/2+1] when half."""
-    _check_cuda_tensor(x)
+    x = _check_cuda_tensor(x)
     H, W = x.shape[-2:]
     batch = x.numel() // (H * W)
     m = W // 2 + 1 if half else W
@@ -421,8 +447,8 @@ def rfft2(x, half: bool = False, out=None):
 
 def rfft2_2x(a, b):
     """RealFFT2D<T>::forward_2x (FFTReal.h:114-118): 2D FFT of a + i b."""
-    _check_cuda_tensor(a, "a")
-    _check_cuda_tensor(b, "b")
+    a = _check_cuda_tensor(a, "a")
+    b = _check_cuda_tensor(b, "b")
     H, W = a.shape
     out = torch.empty(H, W, dtype=_cdtype_for_real(a), device=a.device)
     _check(lib().gfft_real_fft2d_forward_2x(_dtype_code(a), W, H, out.data_ptr(), W, a.data_ptr(), W,
@@ -453,15 +479,18 @@ class RaggedPlan:
         self.offsets = offs
 
     def exec(self, out, x, inverse: bool = False, stream=None):
+        x, _ = _resolved(x, stream), _stored(out)
         _check(lib().gfft_ragged_exec(self._h, int(inverse), out.data_ptr(), x.data_ptr(), _stream_ptr(stream)))
         return out
 
     def adjoint(self, out, g, inverse: bool = False, stream=None):
+        g, _ = _resolved(g, stream), _stored(out)
         _check(lib().gfft_ragged_exec_adjoint(self._h, int(inverse), out.data_ptr(), g.data_ptr(),
                                               _stream_ptr(stream)))
         return out
 
     def autotune(self, out, x, stream=None):
+        x, _ = _resolved(x, stream), _stored(out)
         params = (_I * 3)()
         ms = ctypes.c_double()
         _check(lib().gfft_ragged_autotune(self._h, out.data_ptr(), x.data_ptr(), _stream_ptr(stream), params,

@@ -15,7 +15,7 @@ from collections import OrderedDict
 
 import torch
 
-from . import F32, F64, FLAG_HALF_SPECTRUM, KIND_C2C, KIND_R2C, Plan
+from . import F32, F64, FLAG_HALF_SPECTRUM, KIND_C2C, KIND_R2C, Plan, _dense
 
 _PLANS: "OrderedDict[tuple, Plan]" = OrderedDict()
 _MAX_PLANS = 64
@@ -43,7 +43,7 @@ class FFTFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, inverse: bool = False):
-        x = x.contiguous()
+        x = _dense(x)
         n = x.shape[-1]
         p = _plan(KIND_C2C, _code(x), n, x.numel() // n)
         y = torch.empty_like(x)
@@ -53,7 +53,7 @@ class FFTFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        g = g.contiguous()
+        g = _dense(g)
         n = g.shape[-1]
         p = _plan(KIND_C2C, _code(g), n, g.numel() // n)
         gx = torch.empty_like(g)
@@ -66,7 +66,7 @@ class RFFTFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, half: bool = True):
-        x = x.contiguous()
+        x = _dense(x)
         n = x.shape[-1]
         m = n // 2 + 1 if half else n
         p = _plan(KIND_R2C, _code(x), n, x.numel() // n, FLAG_HALF_SPECTRUM if half else 0)
@@ -78,7 +78,7 @@ class RFFTFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        g = g.contiguous()
+        g = _dense(g)
         n = ctx.n
         p = _plan(KIND_R2C, _code(g), n, g.numel() // g.shape[-1], FLAG_HALF_SPECTRUM if ctx.half else 0)
         rdt = torch.float32 if g.dtype == torch.complex64 else torch.float64
@@ -92,7 +92,7 @@ class IRFFTFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, y, n: int):
-        y = y.contiguous()
+        y = _dense(y)
         p = _plan(KIND_R2C, _code(y), n, y.numel() // y.shape[-1], FLAG_HALF_SPECTRUM)
         rdt = torch.float32 if y.dtype == torch.complex64 else torch.float64
         x = torch.empty(*y.shape[:-1], n, dtype=rdt, device=y.device)
@@ -102,7 +102,7 @@ class IRFFTFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        g = g.contiguous()
+        g = _dense(g)
         n = ctx.n
         p = _plan(KIND_R2C, _code(g), n, g.numel() // n, FLAG_HALF_SPECTRUM)
         cdt = torch.complex64 if g.dtype == torch.float32 else torch.complex128
@@ -136,7 +136,7 @@ class RaggedFFTFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, plan, inverse: bool = False):
-        x = x.contiguous()
+        x = _dense(x)
         y = torch.empty_like(x)
         plan.exec(y, x, inverse)
         ctx.plan, ctx.inverse = plan, inverse
@@ -144,7 +144,7 @@ class RaggedFFTFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        g = g.contiguous()
+        g = _dense(g)
         gx = torch.empty_like(g)
         ctx.plan.adjoint(gx, g, ctx.inverse)
         return gx, None, None

@@ -27,7 +27,7 @@ import torch
 import torch.autograd.forward_ad as _forward_ad
 
 from . import (F32, F64, FLAG_HALF_SPECTRUM, KIND_C2C, KIND_C2C_2D, KIND_R2C, KIND_R2C_2D, KIND_VERT,
-               Plan)
+               Plan, _dense)
 
 __all__ = ["fft", "ifft", "rfft", "irfft", "fft2", "ifft2", "rfft2", "irfft2", "norm_scale"]
 
@@ -107,21 +107,21 @@ def _resize(x, n: int, dim: int):
 # differentiable kernels (last dimension, or last two for 2D)
 
 def _c2c(x, inverse: bool, scale: float):
-    x = x.contiguous()
+    x = _dense(x)
     n = x.shape[-1]
     p = _plan(KIND_C2C, _code(x), n, 0, x.numel() // n)
     return p.exec(torch.empty_like(x), x, inverse, scale=scale)
 
 
 def _c2c2d(x, inverse: bool, scale: float):
-    x = x.contiguous()
+    x = _dense(x)
     h, w = x.shape[-2], x.shape[-1]
     p = _plan(KIND_C2C_2D, _code(x), w, h, x.numel() // (h * w))
     return p.exec(torch.empty_like(x), x, inverse, scale=scale)
 
 
 def _r2c(x, scale: float):
-    x = x.contiguous()
+    x = _dense(x)
     n = x.shape[-1]
     p = _plan(KIND_R2C, _code(x), n, 0, x.numel() // n, FLAG_HALF_SPECTRUM)
     cdt = torch.complex128 if x.dtype == torch.float64 else torch.complex64
@@ -130,7 +130,7 @@ def _r2c(x, scale: float):
 
 
 def _c2r(y, n: int, scale: float):
-    y = y.contiguous()
+    y = _dense(y)
     p = _plan(KIND_R2C, _code(y), n, 0, y.numel() // y.shape[-1], FLAG_HALF_SPECTRUM)
     rdt = torch.float64 if y.dtype == torch.complex128 else torch.float32
     x = torch.empty(*y.shape[:-1], n, dtype=rdt, device=y.device)
@@ -168,7 +168,7 @@ class _R2C(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        g = g.contiguous()
+        g = _dense(g)
         n = ctx.n
         p = _plan(KIND_R2C, _code(g), n, 0, g.numel() // g.shape[-1], FLAG_HALF_SPECTRUM)
         rdt = torch.float64 if g.dtype == torch.complex128 else torch.float32
@@ -184,7 +184,7 @@ class _C2R(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        g = g.contiguous()
+        g = _dense(g)
         n = ctx.n
         p = _plan(KIND_R2C, _code(g), n, 0, g.numel() // n, FLAG_HALF_SPECTRUM)
         cdt = torch.complex128 if g.dtype == torch.float64 else torch.complex64
@@ -316,7 +316,7 @@ def rfft2(input, s=None, dim=(-2, -1), norm=None):
     h, w = x.shape[d0], x.shape[d1]
     _check_pow2(h, "s[0]")
     _check_pow2(w, "s[1]")
-    x = _last2(x, d0, d1).contiguous()
+    x = _dense(_last2(x, d0, d1))
     batch = x.numel() // (h * w)
     p = _plan(KIND_R2C_2D, _code(x), w, h, batch, FLAG_HALF_SPECTRUM)
     cdt = torch.complex128 if x.dtype == torch.float64 else torch.complex64
@@ -339,7 +339,7 @@ def irfft2(input, s=None, dim=(-2, -1), norm=None):
     _check_pow2(h, "s[0]")
     _check_pow2(w, "s[1]")
     m = w // 2 + 1
-    y = _last2(_resize(_resize(y, h, d0), m, d1), d0, d1).contiguous()
+    y = _dense(_last2(_resize(_resize(y, h, d0), m, d1), d0, d1))
     batch = y.numel() // (h * m)
     cols = _plan(KIND_VERT, _code(y), h, m, batch)
     t = torch.empty_like(y)
