@@ -1,8 +1,13 @@
 // fused_tma.cu -- fp32 C2C, R2C and half-spectrum C2R whose complex length is
-// 2^12 .. 2^14, dense and on 16-byte boundaries: the arithmetic of k_c2c_fused,
-// k_r2c_fused and k_c2r_fused (32 points a thread) in a persistent kernel that
-// copies a group's next transform in while it stores this one, and keeps the
-// per-thread twiddles in tensor memory.
+// 2^13 or 2^14, dense and on 16-byte boundaries: the arithmetic of k_c2c_fused,
+// k_r2c_fused and k_c2r_fused (32 points a thread), bit for bit, in a persistent
+// kernel that copies a group's next transform in while it stores this one, and
+// keeps the per-thread twiddles in tensor memory.  Not at 2^12: the plain
+// kernels hold 16 points a thread there, and a transform's bits may not depend
+// on how many others stand beside it (host buffers go through in chunks).  With
+// 32 points the plain kernels are 7 - 20 % slower at 2^12 (GB300, us, 16 / 32
+// points: C2C x 152 3.3 / 3.9, x 4096 46.4 / 51.3; R2C x 2000 30.0 / 33.6),
+// which is more than the persistent kernel gains (C2C x 16384 171.4 / 169.4).
 //
 // What bounded the plain kernels at these lengths is the last pass: its table
 // (31 / 32 of N values, 65 KB at 2^13, 129 KB at 2^14) is read once a
@@ -13,11 +18,10 @@
 // shared memory, which tcgen05.st fills once and tcgen05.ld reads back 16
 // twiddles at a time.  The real transforms' adjustment twiddles (dit.cuh)
 // lie beside them.  GB300, GB/s, C2C, 1 GB batches: 2^14 5616 with tensor
-// memory, 5110 without it, 3994 the plain kernel; 2^13 6246 / 5044 / 4807;
-// 2^12 6633 against 6333 (16 points a thread).  64 points a thread: 4498 at
-// 2^14, 4506 at 2^13.  Real transforms, n = 2^13 / 2^14 / 2^15,
-// 512 MB - 1 GB: R2C 5747 / 4896 / 4130 against 5140 / 4032 / 3453, C2R 5866 /
-// 5293 / 4945 against 5026 / 3730 / 2982.
+// memory, 5110 without it, 3994 the plain kernel; 2^13 6246 / 5044 / 4807.
+// 64 points a thread: 4498 at 2^14, 4506 at 2^13.  Real transforms, n = 2^14 /
+// 2^15, 512 MB - 1 GB: R2C 4896 / 4130 against 4032 / 3453, C2R 5293 / 4945
+// against 3730 / 2982.
 //
 // Replaces FFT<float>::transform<inv> (fft.h:80-85) and RealFFT<float>::forward
 // (FFTReal.h:186-221) for these lengths.
@@ -289,26 +293,19 @@ struct Entry {
     int groups;
     size_t smem[3];     // by kind
 };
-// (packed: 2^13 and 2^14 only, see ragged.cu)
-template <int LOGN, int NG, bool INV>
-const void *packed_fn()
-{
-    if constexpr (LOGN > 12) return (const void *)&k_fused_tma<LOGN, NG, FUSED_C2C, INV, true>;
-    else return nullptr;
-}
 template <int LOGN, int NG>
 Entry make_entry()
 {
     return Entry{{(const void *)&k_fused_tma<LOGN, NG, FUSED_C2C, false>, (const void *)&k_fused_tma<LOGN, NG, FUSED_C2C, true>,
                   (const void *)&k_fused_tma<LOGN, NG, FUSED_R2C, false>, (const void *)&k_fused_tma<LOGN, NG, FUSED_C2R, true>,
-                  packed_fn<LOGN, NG, false>(), packed_fn<LOGN, NG, true>()},
+                  (const void *)&k_fused_tma<LOGN, NG, FUSED_C2C, false, true>, (const void *)&k_fused_tma<LOGN, NG, FUSED_C2C, true, true>},
                  NG,
                  {FusedTmaCfg<LOGN, NG, FUSED_C2C>::SMEM, FusedTmaCfg<LOGN, NG, FUSED_R2C>::SMEM,
                   FusedTmaCfg<LOGN, NG, FUSED_C2R>::SMEM}};
 }
 const Entry &entry(int logn)
 {
-    static const Entry tab[3] = {make_entry<12, 4>(), make_entry<13, 2>(), make_entry<14, 1>()};
+    static const Entry tab[2] = {make_entry<13, 2>(), make_entry<14, 1>()};
     return tab[logn - FUSED_TMA_MIN];
 }
 
@@ -332,8 +329,7 @@ cudaError_t launch(int logn, int kind, int fn_i, const void *in, void *out, long
 
 size_t fused_tma_twiddle_count(int logn)
 {
-    return logn == 12 ? (size_t)StockhamPlan<float, 12, 32>::TW
-         : logn == 13 ? (size_t)StockhamPlan<float, 13, 32>::TW : (size_t)StockhamPlan<float, 14, 32>::TW;
+    return logn == 13 ? (size_t)StockhamPlan<float, 13, 32>::TW : (size_t)StockhamPlan<float, 14, 32>::TW;
 }
 template <int L>
 static void fill(void *buf)
@@ -342,20 +338,17 @@ static void fill(void *buf)
         forward_root<float>(k, M, &w->x, &w->y);
     });
 }
-void fused_tma_twiddle_fill(int logn, void *buf) { (logn == 12 ? fill<12> : logn == 13 ? fill<13> : fill<14>)(buf); }
+void fused_tma_twiddle_fill(int logn, void *buf) { (logn == 13 ? fill<13> : fill<14>)(buf); }
 
 // The persistent kernels pay for filling tensor memory once a CTA and want
-// transforms to reuse it: more than one wave of the SMs at 2^14, three at 2^13,
-// six at 2^12 (C2C, whose plain kernel holds 16 points a thread there and is
-// near the copy rate: twelve).  GB300, us, plain / persistent: C2C 2^14 x 152
-// 12.9 / 13.2, x 304 24.2 / 22.7; 2^13 x 608 21.4 / 21.7, x 1000 33.9 / 32.7;
-// 2^12 x 4096 47.4 / 47.2, x 16384 171.4 / 169.4; R2C of 2^14 reals x 1000
-// 39.9 / 39.7, x 1501 55.5 / 50.9; of 2^13 x 1501 24.0 / 27.1, x 4096
-// 56.9 / 55.0; C2R of 2^13 x 1501 26.3 / 27.1, x 4096 59.8 / 54.5.
-bool fused_tma_takes(int logn, bool real, long long batch)
+// transforms to reuse it: more than one wave of the SMs at 2^14, three at 2^13.
+// GB300, us, plain / persistent: C2C 2^14 x 152 12.9 / 13.2, x 304 24.2 / 22.7;
+// 2^13 x 608 21.4 / 21.7, x 1000 33.9 / 32.7; R2C of 2^14 reals x 1000
+// 39.9 / 39.7, x 1501 55.5 / 50.9.
+bool fused_tma_takes(int logn, long long batch)
 {
     if (logn < FUSED_TMA_MIN || logn > FUSED_TMA_MAX || batch >= (1LL << 30)) return false;
-    const int waves = logn == 14 ? 1 : logn == 13 ? 3 : real ? 6 : 12;
+    const int waves = logn == 14 ? 1 : 3;
     return batch > waves * entry(logn).groups * (long long)sm_count();
 }
 

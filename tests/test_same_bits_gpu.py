@@ -1,0 +1,52 @@
+"""A transform's bits do not depend on what stands beside it: a batch, its
+parts and the host-buffer calls (which go through the device in chunks) give
+the same rows, whichever kernels their sizes select."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def same(a, b):
+    import torch
+    return torch.equal(torch.view_as_real(a) if a.is_complex() else a, torch.view_as_real(b) if b.is_complex() else b)
+
+
+@pytest.mark.parametrize("logn,batch", [(11, 9001), (12, 9001), (13, 1501), (14, 305)])
+def test_c2c_rows(gfft, logn, batch):
+    import torch
+    n = 1 << logn
+    x = torch.randn(batch, n, dtype=torch.complex64, device="cuda")
+    p, one = gfft.Plan(gfft.KIND_C2C, gfft.F32, n, 0, batch), gfft.Plan(gfft.KIND_C2C, gfft.F32, n, 0, 3)
+    for inv in (False, True):
+        y = p.exec(torch.empty_like(x), x, inv)
+        for k in (0, batch // 2, batch - 3):
+            assert same(one.exec(torch.empty_like(x[:3]), x[k:k + 3], inv), y[k:k + 3])
+        odd = torch.empty(batch * n + 1, dtype=torch.complex64, device="cuda")[1:].view(batch, n)
+        odd.copy_(x)  # off a 16-byte boundary
+        assert same(p.exec(torch.empty_like(x), odd, inv), y)
+    hx = x.cpu()
+    for pin in (False, True):
+        src, dst = (t.pin_memory() if pin else t for t in (hx.clone(), torch.zeros_like(hx)))
+        p.exec_host_ptr(dst.data_ptr(), src.data_ptr(), True)
+        assert same(dst, y.cpu())
+
+
+@pytest.mark.parametrize("logn,batch", [(12, 9001), (13, 5001), (14, 1501), (15, 401)])
+def test_real_rows(gfft, logn, batch):
+    import torch
+    n, m = 1 << logn, (1 << (logn - 1)) + 1
+    x = torch.randn(batch, n, device="cuda")
+    f = torch.randn(batch, m, dtype=torch.complex64, device="cuda")
+    p = gfft.Plan(gfft.KIND_R2C, gfft.F32, n, 0, batch, gfft.FLAG_HALF_SPECTRUM)
+    one = gfft.Plan(gfft.KIND_R2C, gfft.F32, n, 0, 3, gfft.FLAG_HALF_SPECTRUM)
+    y, z = torch.empty_like(f), torch.empty_like(x)
+    for call, args, out in (("exec", (x, False), y), ("exec", (f, True), z), ("adjoint", (f, False), z),
+                            ("adjoint", (x, True), y)):
+        getattr(p, call)(out, *args)
+        for k in (0, batch - 3):
+            part = getattr(one, call)(torch.empty_like(out[:3]), args[0][k:k + 3].clone(), args[1])
+            assert same(part, out[k:k + 3]), (call, args[1])
+    p.exec(y, x)
+    hx, hy = x.cpu(), torch.zeros(batch, m, dtype=torch.complex64)
+    p.exec_host_ptr(hy.data_ptr(), hx.data_ptr())
+    assert same(hy, y.cpu())
