@@ -417,15 +417,11 @@ void C2CCore::run_stalled(const void *in, void *out, cudaStream_t st) const
 // ---------------------------------------------------------------------------
 // column FFTs
 
-// columns a tile of TILE_COL_SMALL
-static constexpr int SMALL_C = 4;
-
 void ColCore::init(int dtype_, int logl_, int variant_, bool allow_split, long long max_cols)
 {
     dtype = dtype_;
     logl = logl_;
     variant = variant_;
-    real2d = !allow_split;
     // Columns of up to 2^12 points run in one launch of tiles.  Longer ones
     // (the reference's FFTVert goes to 2^23 rows, fft_impl_generic.h:281-315)
     // run split; fp32 plain columns of 2^10 .. 2^12 also do on request
@@ -475,8 +471,9 @@ void ColCore::init(int dtype_, int logl_, int variant_, bool allow_split, long l
     if (!c) fail(GFFT_ERR_UNSUPPORTED, "no column kernel for this length");
     k = tile_find(dtype, variant, logl, c);
     tw = tile_table(dtype, k, logl, c);
-    if (variant == TILE_COL_PLAIN && (ks = tile_find(dtype, TILE_COL_SMALL, logl, SMALL_C)))
-        tw_s = tile_table(dtype, ks, logl, SMALL_C);
+    for (int i = 0; i < 2 && variant == TILE_COL_PLAIN; i++)
+        if ((narrow[i].k = tile_find(dtype, TILE_COL_SMALL, logl, 2 << i)))
+            narrow[i].tw = tile_table(dtype, narrow[i].k, logl, 2 << i);
 }
 
 void ColCore::release()
@@ -485,26 +482,38 @@ void ColCore::release()
     scratch = nullptr;
 }
 
+// The narrow tiles run the radices of the pipelined ones (a column's bits do
+// not depend on how many stand beside it), with plain loads.  They finish
+// sooner while few CTAs of the pipelined tiles would be at work, or, at 2^12,
+// while the columns are few and every row's 48-byte box carries 32 bytes.
+// GB300, us a call, pipelined / 4 columns / 2 columns:
+//   2^11  8 columns 7.4 / 5.2 / 5.2, 64 7.5 / 7.0 / 7.2, 192 7.5 / 7.6 / 9.1; off
+//         16 bytes 17 10.3 / 7.0 / 6.6, 129 10.3 / 7.8 / 7.4, 305 10.3 / 10.0 / 11.0,
+//         513 10.4 / 13.5 / 18.7; 144 in 16 images, in place, 14.2 / 17.4 / 21.9
+//   2^12  1 column 9.6 / 7.4 / 4.8, 8 8.6 / 9.1 / 7.6, 16 9.2 / 10.7 / 10.8; off 16
+//         bytes 257 12.6 / 12.1 / 21.0, 607 16.1 / 13.9 / 30.7, 609 21.6 / 22.0
+// (16 points a thread, which they held before: 64 of 2^11 6.5, 129 6.5, 607 6.7)
+const TileKernel *ColCore::tile_for(long long cols, bool odd, int *width, const void **table) const
+{
+    const long long sms = sm_count();
+    const bool two = cols <= (logl == 11 && odd ? 64 : 8);
+    const bool four = logl == 11 ? cols <= sms : odd && cols <= 4 * sms;
+    const int i = narrow[0].k && two ? 0 : narrow[1].k && four ? 1 : -1;
+    *width = i < 0 ? c : 2 << i;
+    *table = i < 0 ? tw : narrow[i].tw;
+    return i < 0 ? k : narrow[i].k;
+}
+
 void ColCore::run(int inverse, const void *in, void *out, long long ncols, long long ld_in, long long ld_out,
                   long long batch, long long idist, long long odist, cudaStream_t st, double scale) const
 {
-    // The 4-column tiles of 16 points a thread:
-    // - few columns: while these tiles run in one wave of the 152 SMs they
-    //   finish sooner than the wide tiles of 64 points a thread (GB300, us a
-    //   call: 256 columns of 2^11 points 7.1 against 8.6, of 2^12 11.8 /
-    //   12.2; 1024 columns 13.5 / 11.6 and 24.0 / 23.6);
-    // - the column pass of real 2D transforms at 2^12, whatever its stride
-    //   (half- and full-width results hold the same bits), and 2^12 rows off
-    //   16-byte boundaries while the columns stay in L2 (96 of 129 MB):
-    //   boxes of 48 bytes for runs of 32 lose there what the copies gain
-    //   (real 4096 x 4096, forward and back, 166 us against 169 - 195).
-    //   Out of HBM the copies win: 4001 columns 88 us against 117.
     if (!split) {
         const bool odd = ((uintptr_t)in & 15u) != 0 || ld_in % 2 != 0;
-        const bool few = ks && (ncols * batch <= 152 * SMALL_C || (logl == 12 && (real2d || (odd && ((ncols * batch) << 15) <= (96LL << 20)))));
-        const int cw = few ? SMALL_C : c;
-        check_cuda(launch_colpass(few ? *ks : *k, inverse, (ncols + cw - 1) / cw, batch, in, out, ncols, ld_in, ld_out,
-                                  idist, odist, few ? tw_s : tw, nullptr, nullptr, 0, 0u, st, scale),
+        int cw;
+        const void *table;
+        const TileKernel *tile = tile_for(ncols * batch, odd, &cw, &table);
+        check_cuda(launch_colpass(*tile, inverse, (ncols + cw - 1) / cw, batch, in, out, ncols, ld_in, ld_out, idist,
+                                  odist, table, nullptr, nullptr, 0, 0u, st, scale),
                    "launch column FFT");
         if (herm_fill)
             check_cuda(launch_herm_fill(dtype, out, 1LL << logl, 2 * (ncols - 1), ld_out, batch, odist, st),

@@ -68,10 +68,12 @@ struct ColCore {
     int dtype = 0, logl = 0, variant = 0, c = 0;
     const TileKernel *k = nullptr;
     const void *tw = nullptr;
-    // fp32 columns of 2^11 and 2^12 points: the short tile for few columns
-    const TileKernel *ks = nullptr;
-    const void *tw_s = nullptr;
-    bool real2d = false;  // the column pass of a real 2D transform
+    // fp32 columns of 2^11 and 2^12 points: narrow tiles for few columns
+    // (tile_for), of 2 and 4 columns
+    struct Narrow {
+        const TileKernel *k = nullptr;
+        const void *tw = nullptr;
+    } narrow[2];
     // split column FFTs (columns longer than one tile, 2^13 .. 2^24 points,
     // and fp32 plain columns of 2^10 .. 2^12 on request): each column of
     // H = H1 * H2 points is two launches of short column FFTs per band of
@@ -96,6 +98,9 @@ struct ColCore {
         if (!split) return 1 + (herm_fill ? 1 : 0);
         return 2 * batch * ((ncols + band - 1) / band) + (rows_bitrev ? 1 : 0) + (herm_fill ? 1 : 0);
     }
+    // the tile `cols` columns take (its width and table), rows off 16-byte
+    // boundaries or not
+    const TileKernel *tile_for(long long cols, bool odd, int *width, const void **table) const;
     void run(int inverse, const void *in, void *out, long long ncols, long long ld_in, long long ld_out,
              long long batch, long long idist, long long odist, cudaStream_t st, double scale = 1.0) const;
 };

@@ -53,6 +53,7 @@ struct TileReg {
         } else {
             using Cfg = ColCfg<T, LOGL, C, E>;
             constexpr bool tw4 = V == TILE_COL_TW4, br = V == TILE_COL_BITREV, herm = V == TILE_COL_HERM;
+            constexpr bool plain_loads = br || V == TILE_COL_SMALL;
             constexpr int twm = tw4 ? 1 : V == TILE_COL_TWB ? 2 : 0;
             k.fwd = (const void *)&k_colpass<T, LOGL, C, E, false, twm, br, herm>;
             k.inv = (const void *)&k_colpass<T, LOGL, C, E, true, twm, br, herm>;
@@ -60,7 +61,7 @@ struct TileReg {
             k.smem = Cfg::SMEM;
             using TCfg = ColTmaCfg<T, LOGL, C, E>;
             using TCfg1 = ColTmaCfg<T, LOGL, C, E, 1>;
-            if constexpr (!br && TCfg::SMEM <= 220 * 1024 && C * sizeof(cpx<T>) % 16 == 0) {
+            if constexpr (!plain_loads && TCfg::SMEM <= 220 * 1024 && C * sizeof(cpx<T>) % 16 == 0) {
                 k.tma_fwd = (const void *)&k_colpass_tma<T, LOGL, C, E, false, twm, herm>;
                 k.tma_inv = (const void *)&k_colpass_tma<T, LOGL, C, E, true, twm, herm>;
                 k.tma_threads = TCfg::THREADS;

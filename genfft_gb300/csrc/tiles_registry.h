@@ -18,7 +18,7 @@ enum TileVariant {
     TILE_COL_HERM = 4,    // column FFT + Hermitian mirror store (real 2D)
     TILE_COL_TWB = 5,     // column pass with the W_N^(batch * row) twiddle (split column FFTs)
     TILE_COL_TWP = 6,     // TILE_COL_TW4 with 32 or 64 points a thread (tiles_pipe.cuh)
-    TILE_COL_SMALL = 8,   // TILE_COL_PLAIN for few columns (one wave of short tiles)
+    TILE_COL_SMALL = 8,   // TILE_COL_PLAIN for few columns (narrow tiles of plain loads)
     TILE_ROW_PIPE = 7     // TILE_ROW_XPOSE with 32 or 64 points a thread (tiles_pipe.cuh)
 };
 

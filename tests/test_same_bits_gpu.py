@@ -50,3 +50,44 @@ def test_real_rows(gfft, logn, batch):
     hx, hy = x.cpu(), torch.zeros(batch, m, dtype=torch.complex64)
     p.exec_host_ptr(hy.data_ptr(), hx.data_ptr())
     assert same(hy, y.cpu())
+
+
+@pytest.mark.parametrize("logl", [9, 10, 11, 12])
+def test_columns(gfft, logl):
+    """Any columns of any number of columns, whatever the row stride and the
+    boundary the rows start on."""
+    import torch
+    h = 1 << logl
+    x = torch.randn(h, 700, dtype=torch.complex64, device="cuda")
+    whole = gfft.fft_vert(x)
+    for w in (1, 2, 3, 4, 5, 8, 9, 16, 17, 152, 153, 304, 513, 608, 609):
+        assert same(gfft.fft_vert(x[:, :w].contiguous()), whole[:, :w].contiguous()), w
+        p = gfft.Plan(gfft.KIND_VERT, gfft.F32, h, w, 1, 0, 700, 0, 700)
+        y = torch.empty_like(x)
+        p.exec(y[:, 1:], x[:, 1:])
+        assert same(y[:, 1:1 + w].contiguous(), whole[:, 1:1 + w].contiguous()), w
+
+
+@pytest.mark.parametrize("logl,w,batch", [(11, 64, 6), (11, 33, 9), (12, 3, 300), (12, 33, 33), (12, 513, 3)])
+def test_batches_of_columns(gfft, logl, w, batch):
+    import torch
+    h = 1 << logl
+    x = torch.randn(batch, h, w, dtype=torch.complex64, device="cuda")
+    p, one = gfft.Plan(gfft.KIND_VERT, gfft.F32, h, w, batch), gfft.Plan(gfft.KIND_VERT, gfft.F32, h, w, 1)
+    y = p.exec(torch.empty_like(x), x)
+    for b in range(0, batch, 4):
+        assert same(one.exec(torch.empty_like(x[0]), x[b]), y[b]), b
+    hx = x.cpu()
+    hy = torch.zeros_like(hx)
+    p.exec_host_ptr(hy.data_ptr(), hx.data_ptr())
+    assert same(hy, y.cpu())
+
+
+@pytest.mark.parametrize("h,w,batch", [(2048, 64, 12), (4096, 32, 40), (4096, 512, 5)])
+def test_batches_of_real_images(gfft, h, w, batch):
+    import torch
+    x = torch.randn(batch, h, w, device="cuda")
+    half, full = gfft.rfft2(x, half=True), gfft.rfft2(x)
+    assert same(half, full[..., :w // 2 + 1].contiguous())
+    for b in (0, batch - 1):
+        assert same(gfft.rfft2(x[b], half=True), half[b]) and same(gfft.rfft2(x[b]), full[b])
