@@ -135,6 +135,23 @@ __device__ __forceinline__ cpx<T> ldcs_c(const cpx<T> *p)
     auto v = __ldcs(reinterpret_cast<const typename vec2<T>::type *>(p));
     return {v.x, v.y};
 }
+// What an earlier kernel of the stream wrote, in a kernel launch_pdl may have
+// resident while that one still runs: from L2.  Through `const __restrict__` a
+// plain load may take the read-only path, which holds for data that nothing
+// writes while the kernel is there, and its L1 lines may be older than the
+// wait in pdl_enter.
+__device__ __forceinline__ cpx<float> ldcg_c(const cpx<float> *p)
+{
+    cpx<float> v;
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ cpx<double> ldcg_c(const cpx<double> *p)
+{
+    cpx<double> v;
+    asm volatile("ld.global.cg.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
 template <typename T>
 __device__ __forceinline__ void stcs_c(cpx<T> *p, cpx<T> a)
 {

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(RowDitCfg<T, LOGB, CH, E_>::THREADS, 1024 / Ro
     {
         const cpx<T> *src = in + b * idist + k1 * B + t;
 #pragma unroll
-        for (int q = 0; q < E; q++) v[q] = active ? ld_c(src + q * G) : cpx<T>{(T)0, (T)0};
+        for (int q = 0; q < E; q++) v[q] = active ? ldcg_c(src + q * G) : cpx<T>{(T)0, (T)0};
     }
     cpx<T> *my = sm + s * Cfg::ROWP;
     stockham_run<T, LOGB, E_, false>(

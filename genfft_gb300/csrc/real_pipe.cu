@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(C2RColCfg::THREADS, 1)
 #pragma unroll
             for (int q = 0; q < E; q++) {
                 const int a = t + q * G;
-                c32 fk = ld_c(F + (long long)B * a), fp = ld_c(F + (long long)B * (N - a));
+                c32 fk = ldcg_c(F + (long long)B * a), fp = ldcg_c(F + (long long)B * (N - a));
                 if (a == 0) {  // F_0 and F_H count as real, and whole
                     fk.y = 0.f;
                     fp.y = 0.f;

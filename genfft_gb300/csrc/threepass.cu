@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(StockhamPlan<float, L, 16>::G *R, MINB)
     const c32 *src = in + y * idist + k1 * lda + k2 * ldb + t;
     c32 v[E];
 #pragma unroll
-    for (int q = 0; q < E; q++) v[q] = ld_c(src + q * G);
+    for (int q = 0; q < E; q++) v[q] = ldcg_c(src + q * G);
     c32 *const my = sm + s * ROWP;
     stockham_run<float, L, 16, INV>(
         v, t, [my](int i) -> c32 & { return my[spad<float>(i)]; }, tw, []() { __syncthreads(); });

@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(RowCfg<T, LOGL, C, E_>::THREADS)
         cpx<T> v[E];
         const cpx<T> *src = in + b * idist + row * ld_in + t;
 #pragma unroll
-        for (int q = 0; q < E; q++) v[q] = active ? ld_c(src + q * G) : cpx<T>{(T)0, (T)0};
+        for (int q = 0; q < E; q++) v[q] = active ? ldcg_c(src + q * G) : cpx<T>{(T)0, (T)0};
         cpx<T> *my = sm + s * Cfg::ROW;
         stockham_run<T, LOGL, E_, INV>(
             v, t, [my](int i) -> cpx<T> & { return my[spad<T>(i)]; }, tw, []() { __syncthreads(); });
