@@ -347,7 +347,7 @@ void fused_tma_twiddle_fill(int logn, void *buf) { (logn == 13 ? fill<13> : fill
 // 39.9 / 39.7, x 1501 55.5 / 50.9.
 bool fused_tma_takes(int logn, long long batch)
 {
-    if (logn < FUSED_TMA_MIN || logn > FUSED_TMA_MAX || batch >= (1LL << 30)) return false;
+    if (logn < FUSED_TMA_MIN || logn > FUSED_TMA_MAX || batch >= (1LL << 30) || !tma_enabled()) return false;
     const int waves = logn == 14 ? 1 : 3;
     return batch > waves * entry(logn).groups * (long long)sm_count();
 }

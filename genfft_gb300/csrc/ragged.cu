@@ -495,7 +495,7 @@ constexpr long long RAGGED_PIPE_POINTS = 1LL << 23;
 static bool ragged_pipe_takes(int logn, long long count)
 {
     return logn >= RAGGED_PIPE_MIN && logn <= RAGGED_PIPE_MAX && (count << logn) >= RAGGED_PIPE_POINTS &&
-           count < (1LL << 24);
+           count < (1LL << 24) && tensor_maps_enabled();
 }
 // ... or, for 2^13 and 2^14, through the persistent fused kernel: one pass of
 // HBM traffic instead of two, a launch of its own (GB300, us an exec of 2^22 /

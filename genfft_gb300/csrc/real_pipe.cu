@@ -55,7 +55,9 @@ struct RowDitPipeCfg : PipeCfg<float, RL, RC, RE, 2, 2, LAND_ROW> {
     static_assert(SMEM <= 227 * 1024, "fits one CTA");
 };
 
-// in: the column pass's output, rows of 512; out: H + 1 bins a transform
+// in: the column pass's output, rows of 512; out: H + 1 bins a transform.
+// TMA false (GFFT_NO_TMA): each thread loads its own points.
+template <bool TMA>
 __global__ void __launch_bounds__(RowDitPipeCfg::THREADS, 1)
     k_rowdit_pipe(const c32 *__restrict__ in, c32 *__restrict__ out, int A, long long idist, long long odist,
                   int nbatch, const c32 *__restrict__ tw, const c32 *__restrict__ dtw, unsigned *err, float scale)
@@ -92,7 +94,7 @@ __global__ void __launch_bounds__(RowDitPipeCfg::THREADS, 1)
 
     auto issue = [&](int i) {
         const int w = w0 + i * step;
-        if (w >= total) return;
+        if (!TMA || w >= total) return;
         const int buf = i % NB;
         c32 *const S = stage0 + (size_t)buf * Cfg::STAGE;
         const int b = (int)((unsigned)w / (unsigned)tiles), p = w - b * tiles;
@@ -113,18 +115,26 @@ __global__ void __launch_bounds__(RowDitPipeCfg::THREADS, 1)
         const int k1 = row0 ? 0 : s < 8 ? 1 + 8 * p + s : A - 1 - 8 * p - (s - 8);
         // t_k of this thread's point 0 (bins k1 + A (t + G q))
         const c32 t0 = ldg_c(dtw + k1 + (long long)A * t);
-        const bool ok = stage_wait(&full[buf], &seq[buf], i, par);
+        const bool ok = TMA ? stage_wait(&full[buf], &seq[buf], i, par) : true;
         const bool active = !row0 || s == 0;
         c32 v[E];
+        if constexpr (TMA) {
 #pragma unroll
-        for (int q = 0; q < E; q++) v[q] = active ? S[s * Cfg::RP + t + q * G] : c32{0.f, 0.f};
+            for (int q = 0; q < E; q++) v[q] = active ? S[s * Cfg::RP + t + q * G] : c32{0.f, 0.f};
+        } else {
+            const c32 *const row = in + (long long)b * idist + (long long)k1 * N;
+#pragma unroll
+            for (int q = 0; q < E; q++) v[q] = active ? ldcg_c(row + t + q * G) : c32{0.f, 0.f};
+        }
         bool landed = true;
         c32 *const my = S + s * Cfg::PITCH;
         stockham_run<float, RL, RE, false, TwShared>(
             v, t, [my](int k) -> c32 & { return my[Cfg::padded(k)]; }, tws, [bar]() { bar_group(bar, GT); },
             [&]() {
-                stage_read(bar + 1, GT, tid);
-                stage_refill(bar + 1, GT, tid, landed, i + NB, issue);
+                if constexpr (TMA) {
+                    stage_read(bar + 1, GT, tid);
+                    stage_refill(bar + 1, GT, tid, landed, i + NB, issue);
+                }
             },
             [&]() { landed = bar_group_and(bar, GT, ok); });
         if (!landed) return false;
@@ -182,7 +192,9 @@ struct C2RColCfg : PipeCfg<float, RL, RC, RE, 2, 2, LAND_ROW> {
 // transforms as [512 rows][B], rounded down to 16 bytes; bit r of skew: those
 // of parity r start 8 bytes in); out: the workspace, rows of B.
 // interior = 0.5: the adjoint of the half-spectrum R2C halves every bin but
-// F_0 and F_H.
+// F_0 and F_H.  TMA false (GFFT_NO_TMA, or no tensor map for this input): each
+// thread loads its own bins.
+template <bool TMA>
 __global__ void __launch_bounds__(C2RColCfg::THREADS, 1)
     k_c2rcol_pipe(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap map1, int skew,
                   const c32 *__restrict__ in, long long idist, c32 *__restrict__ out, int B, int nbatch,
@@ -224,7 +236,7 @@ __global__ void __launch_bounds__(C2RColCfg::THREADS, 1)
     auto hi_x = [&](int b, int p) { return B - 8 - 8 * p + (skew >> (b & 1) & 1); };
     auto issue = [&](int i) {
         const int w = w0 + i * step;
-        if (w >= total) return;
+        if (!TMA || w >= total) return;
         const int buf = i % NB;
         c32 *const S = stage0 + (size_t)buf * Cfg::STAGE;
         const int b = (int)((unsigned)w / (unsigned)tiles), p = w - b * tiles;
@@ -259,7 +271,7 @@ __global__ void __launch_bounds__(C2RColCfg::THREADS, 1)
             const int cl = col0 ? 0 : sl < 8 ? 1 + 8 * p + sl : B - 1 - 8 * p - (sl - 8);
             cp_async8(t2s + idx, t2 + cl * E + q);
         }
-        const bool ok = stage_wait(&full[buf], &seq[buf], i, par);
+        const bool ok = TMA ? stage_wait(&full[buf], &seq[buf], i, par) : true;
         c32 v[E];
         if (!col0) {
             // own column and its mirror: element a pairs with N - 1 - a
@@ -269,26 +281,45 @@ __global__ void __launch_bounds__(C2RColCfg::THREADS, 1)
             static_for<0, E>([&](auto qc) {
                 constexpr int q = decltype(qc)::value;
                 const int a = t + q * G;
-                const c32 fk = S[own + a * CBW], fp = S[mir + (N - 1 - a) * CBW];
+                c32 fk, fp;
+                if constexpr (TMA) {
+                    fk = S[own + a * CBW];
+                    fp = S[mir + (N - 1 - a) * CBW];
+                } else {
+                    const long long k = (long long)B * a + col;
+                    fk = ldcg_c(in + (long long)b * idist + k);
+                    fp = ldcg_c(in + (long long)b * idist + (H - k));
+                }
                 const c32 sm{fk.x + fp.x, fk.y - fp.y};   // F_k + conj F_p
                 const c32 df{fp.x - fk.x, -fp.y - fk.y};  // conj F_p - F_k
                 const c32 m = cmulc(df, rot64<q, false, float>(t0));
                 v[q] = c32{(sm.x + m.x) * interior, (sm.y + m.y) * interior};
             });
         } else if (active) {
+            // (eight pairs of bins in flight a thread)
             const c32 *F = in + (long long)b * idist;
+            constexpr int CH = 8;
 #pragma unroll
-            for (int q = 0; q < E; q++) {
-                const int a = t + q * G;
-                c32 fk = ldcg_c(F + (long long)B * a), fp = ldcg_c(F + (long long)B * (N - a));
-                if (a == 0) {  // F_0 and F_H count as real, and whole
-                    fk.y = 0.f;
-                    fp.y = 0.f;
+            for (int q0 = 0; q0 < E; q0 += CH) {
+                c32 fk[CH], fp[CH];
+#pragma unroll
+                for (int j = 0; j < CH; j++) {
+                    const long long a = t + (q0 + j) * G;
+                    fk[j] = ldcg_c(F + B * a);
+                    fp[j] = ldcg_c(F + B * (N - a));
                 }
-                const float f = a == 0 ? 1.f : interior;
-                const c32 sm{fk.x + fp.x, fk.y - fp.y}, df{fp.x - fk.x, -fp.y - fk.y};
-                const c32 m = cmulc(df, ldg_c(dtw + (long long)B * a));
-                v[q] = c32{(sm.x + m.x) * f, (sm.y + m.y) * f};
+#pragma unroll
+                for (int j = 0; j < CH; j++) {
+                    const int a = t + (q0 + j) * G;
+                    if (a == 0) {  // F_0 and F_H count as real, and whole
+                        fk[j].y = 0.f;
+                        fp[j].y = 0.f;
+                    }
+                    const float f = a == 0 ? 1.f : interior;
+                    const c32 sm{fk[j].x + fp[j].x, fk[j].y - fp[j].y}, df{fp[j].x - fk[j].x, -fp[j].y - fk[j].y};
+                    const c32 m = cmulc(df, ldg_c(dtw + (long long)B * a));
+                    v[q0 + j] = c32{(sm.x + m.x) * f, (sm.y + m.y) * f};
+                }
             }
         } else {
 #pragma unroll
@@ -299,8 +330,10 @@ __global__ void __launch_bounds__(C2RColCfg::THREADS, 1)
         stockham_run<float, RL, RE, true, TwShared>(
             v, t, [my](int k) -> c32 & { return my[Cfg::padded(k)]; }, tws, [bar]() { bar_group(bar, GT); },
             [&]() {
-                stage_read(bar + 1, GT, tid);
-                stage_refill(bar + 1, GT, tid, landed, i + NB, issue);
+                if constexpr (TMA) {
+                    stage_read(bar + 1, GT, tid);
+                    stage_refill(bar + 1, GT, tid, landed, i + NB, issue);
+                }
             },
             [&]() {
                 cp_async_wait();
@@ -337,7 +370,7 @@ void realpipe_twiddle_fill(void *buf)
 cudaError_t launch_rowdit_pipe(const void *in, void *out, long long A, long long batch, long long idist,
                                long long odist, const void *tw, const void *dtw, cudaStream_t st, double scale)
 {
-    const void *fn = (const void *)&k_rowdit_pipe;
+    const void *fn = tma_enabled() ? (const void *)&k_rowdit_pipe<true> : (const void *)&k_rowdit_pipe<false>;
     cudaError_t e = ensure_smem(fn, RowDitPipeCfg::SMEM);
     if (e != cudaSuccess) return e;
     int a = (int)A, nb = (int)batch;
@@ -352,13 +385,11 @@ cudaError_t launch_rowdit_pipe(const void *in, void *out, long long A, long long
 cudaError_t launch_c2rcol_pipe(const void *in, void *ws, long long B, long long batch, long long idist, const void *tw,
                                const void *t1, const void *t2, const void *dtw, bool half_interior, cudaStream_t st)
 {
-    const void *fn = (const void *)&k_c2rcol_pipe;
-    cudaError_t e = ensure_smem(fn, C2RColCfg::SMEM);
-    if (e != cudaSuccess) return e;
-    CUtensorMap map[2];
+    CUtensorMap map[2] = {};
     int skew = 0;
     constexpr int N = C2RColCfg::N;
-    for (int r = 0; r < 2; r++) {
+    bool tma = tensor_maps_enabled();
+    for (int r = 0; r < 2 && tma; r++) {
         if (r == 1 && batch == 1) {
             map[1] = map[0];
             break;
@@ -366,11 +397,13 @@ cudaError_t launch_c2rcol_pipe(const void *in, void *ws, long long B, long long 
         const uintptr_t base = (uintptr_t)in + (uintptr_t)(r * idist) * sizeof(c32);
         const int off = (int)(base >> 3 & 1);
         skew |= off << r;
-        if (!make_tensor_map_3d(&map[r], (const void *)(base & ~(uintptr_t)15), (unsigned long long)(B + off), N,
-                                (unsigned long long)((batch + 1 - r) / 2), (unsigned long long)B * sizeof(c32),
-                                (unsigned long long)(2 * idist) * sizeof(c32), CBW, C2RColCfg::BOXR))
-            return cudaErrorInvalidValue;
+        tma = make_tensor_map_3d(&map[r], (const void *)(base & ~(uintptr_t)15), (unsigned long long)(B + off), N,
+                                 (unsigned long long)((batch + 1 - r) / 2), (unsigned long long)B * sizeof(c32),
+                                 (unsigned long long)(2 * idist) * sizeof(c32), CBW, C2RColCfg::BOXR);
     }
+    const void *fn = tma ? (const void *)&k_c2rcol_pipe<true> : (const void *)&k_c2rcol_pipe<false>;
+    cudaError_t e = ensure_smem(fn, C2RColCfg::SMEM);
+    if (e != cudaSuccess) return e;
     int b = (int)B, nb = (int)batch;
     float interior = half_interior ? 0.5f : 1.0f;
     unsigned *err = device_error_word();

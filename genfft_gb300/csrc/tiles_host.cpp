@@ -77,16 +77,16 @@ cudaError_t launch_pdl(const void *fn, dim3 grid, dim3 block, void **args, size_
     return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
-namespace {
-
-bool tma_disabled()
+bool tma_enabled()
 {
-    static const bool off = [] {
+    static const bool on = [] {
         const char *v = std::getenv("GFFT_NO_TMA");
-        return v && *v && *v != '0';
+        return !(v && *v && *v != '0');
     }();
-    return off;
+    return on;
 }
+
+namespace {
 
 // single-buffered TMA tile kernels: GFFT_TMA1 unset or 1 = used (row and
 // column passes), 2 = column passes only, 0 = not used
@@ -101,7 +101,7 @@ static int tma1_mode()
 
 static bool use_tma(const TileKernel &k)
 {
-    if (!k.tma_fwd || tma_disabled()) return false;
+    if (!k.tma_fwd || !tma_enabled()) return false;
     if (k.tma_stages != 1) return true;
     const int m = tma1_mode();
     return m == 1 || (m == 2 && !k.tma_row);
@@ -151,6 +151,8 @@ long long persistent_grid(const void *fn, int threads, size_t smem, long long wo
 }
 
 }  // namespace
+
+bool tensor_maps_enabled() { return tma_enabled() && encode_fn(); }
 
 bool make_tensor_map_3d(CUtensorMap *map, const void *base, unsigned long long dx, unsigned long long dy,
                         unsigned long long dz, unsigned long long sy_bytes, unsigned long long sz_bytes, unsigned bx,

@@ -74,6 +74,11 @@ bool make_tensor_map_3d(CUtensorMap *map, const void *base, unsigned long long d
                         unsigned long long dz, unsigned long long sy_bytes, unsigned long long sz_bytes, unsigned bx,
                         unsigned by);
 
+// whether the kernels that copy with TMA may be used at all (GFFT_NO_TMA), and
+// whether tensor maps can be made too (the driver has their encoder)
+bool tma_enabled();
+bool tensor_maps_enabled();
+
 // SMs of the current device
 int sm_count();
 
