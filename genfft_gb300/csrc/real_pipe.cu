@@ -188,6 +188,17 @@ struct C2RColCfg : PipeCfg<float, RL, RC, RE, 2, 2, LAND_ROW> {
     static_assert(SMEM <= 227 * 1024, "fits one CTA");
 };
 
+// Z'_k from bins k and H - k weighted by f, 1 or 1/2 (c2r.cu).  The weight
+// comes first, in the adds' multiply-adds: the sum of two bins may overflow
+// where that of their halves does not.
+__device__ __forceinline__ c32 c2r_value(c32 fk, c32 fp, c32 tk, float f)
+{
+    const c32 h = scl(fp, f);
+    const c32 sm{fma_(fk.x, f, h.x), fma_(fk.y, f, -h.y)};   // F_k + conj F_p
+    const c32 df{fma_(-fk.x, f, h.x), fma_(-fk.y, f, -h.y)};  // conj F_p - F_k
+    return sm + cmulc(df, tk);
+}
+
 // in: H + 1 bins a transform, H = 512 B (map / map1: the even / odd
 // transforms as [512 rows][B], rounded down to 16 bytes; bit r of skew: those
 // of parity r start 8 bytes in); out: the workspace, rows of B.
@@ -290,10 +301,7 @@ __global__ void __launch_bounds__(C2RColCfg::THREADS, 1)
                     fk = ldcg_c(in + (long long)b * idist + k);
                     fp = ldcg_c(in + (long long)b * idist + (H - k));
                 }
-                const c32 sm{fk.x + fp.x, fk.y - fp.y};   // F_k + conj F_p
-                const c32 df{fp.x - fk.x, -fp.y - fk.y};  // conj F_p - F_k
-                const c32 m = cmulc(df, rot64<q, false, float>(t0));
-                v[q] = c32{(sm.x + m.x) * interior, (sm.y + m.y) * interior};
+                v[q] = c2r_value(fk, fp, rot64<q, false, float>(t0), interior);
             });
         } else if (active) {
             // (eight pairs of bins in flight a thread)
@@ -315,10 +323,7 @@ __global__ void __launch_bounds__(C2RColCfg::THREADS, 1)
                         fk[j].y = 0.f;
                         fp[j].y = 0.f;
                     }
-                    const float f = a == 0 ? 1.f : interior;
-                    const c32 sm{fk[j].x + fp[j].x, fk[j].y - fp[j].y}, df{fp[j].x - fk[j].x, -fp[j].y - fk[j].y};
-                    const c32 m = cmulc(df, ldg_c(dtw + (long long)B * a));
-                    v[q0 + j] = c32{(sm.x + m.x) * f, (sm.y + m.y) * f};
+                    v[q0 + j] = c2r_value(fk[j], fp[j], ldg_c(dtw + (long long)B * a), a == 0 ? 1.f : interior);
                 }
             }
         } else {
