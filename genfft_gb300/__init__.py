@@ -295,7 +295,9 @@ def fft(x, inverse: bool = False, out=None):
     batch = x.numel() // n if n else 0
     if out is None:
         out = torch.empty_like(x)
-    _check(lib().gfft_fft_transform(_dtype_code(x), n, batch, int(inverse), _stored(out).data_ptr(),
+    else:
+        _stored(out)
+    _check(lib().gfft_fft_transform(_dtype_code(x), n, batch, int(inverse), out.data_ptr(),
                                     x.data_ptr(), _stream_ptr()))
     return out
 
@@ -404,8 +406,10 @@ def fft_vert(x, inverse: bool = False, out=None):
     rows, cols = x.shape
     if out is None:
         out = torch.empty_like(x)
-    _check(lib().gfft_vert_transform(_dtype_code(x), rows, int(inverse), _stored(out).data_ptr(), cols,
-                                     x.data_ptr(), cols, cols, _stream_ptr()))
+    else:
+        _stored(out)
+    _check(lib().gfft_vert_transform(_dtype_code(x), rows, int(inverse), out.data_ptr(), cols, x.data_ptr(),
+                                     cols, cols, _stream_ptr()))
     return out
 
 
