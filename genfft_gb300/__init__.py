@@ -16,10 +16,16 @@ import os
 import threading
 from collections import OrderedDict
 
-try:
-    import torch
-except ImportError:  # the ABI itself needs no torch; the tensor functions below do
-    torch = None
+
+class _Torch:
+    """torch, imported when the first tensor function needs it: the ABI itself
+    (lib(), plans on raw pointers, host buffers) works without."""
+
+    def __getattr__(self, name):
+        return getattr(_import_torch(), name)
+
+
+torch = _Torch()
 
 __all__ = ["GFFTError", "Plan", "lib", "lib_path", "fft", "fft_tc", "ifft", "fft_no_scramble", "rfft", "fft_real_input",
            "fft_interleave", "separate_2x", "dit", "fft_vert", "fft_vert_no_scramble", "fft2", "rfft2",
@@ -126,9 +132,23 @@ def _check(status: int) -> None:
         raise GFFTError(status, msg.decode() if msg else "")
 
 
-# the current stream's handle without a Stream object around it (0.1 us
-# against 2.9)
-_raw_stream = getattr(getattr(torch, "_C", None), "_cuda_getCurrentRawStream", None)
+# set by _import_torch: the current stream's handle without a Stream object
+# around it (0.1 us against 2.9), and the dtypes the library takes
+_raw_stream = None
+_CODES: dict = {}
+_COMPLEX: tuple = ()
+_REAL: tuple = ()
+
+
+def _import_torch():
+    global torch, _raw_stream, _CODES, _COMPLEX, _REAL
+    import torch as module
+    _raw_stream = getattr(module._C, "_cuda_getCurrentRawStream", None)
+    _COMPLEX = (module.complex64, module.complex128)
+    _REAL = (module.float32, module.float64)
+    _CODES = {module.complex64: F32, module.float32: F32, module.complex128: F64, module.float64: F64}
+    torch = module
+    return module
 
 
 def _stream_ptr(stream=None) -> int:
@@ -139,13 +159,9 @@ def _stream_ptr(stream=None) -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
-_CODES = {} if torch is None else {torch.complex64: F32, torch.float32: F32, torch.complex128: F64,
-                                   torch.float64: F64}
-_COMPLEX = () if torch is None else (torch.complex64, torch.complex128)
-_REAL = () if torch is None else (torch.float32, torch.float64)
-
-
 def _dtype_code(t) -> int:
+    if not _CODES:
+        _import_torch()
     code = _CODES.get(t.dtype)
     if code is None:
         raise TypeError(f"unsupported dtype {t.dtype}")
@@ -278,6 +294,8 @@ def device_error() -> int:
 
 
 def _check_cuda_tensor(x, name="x"):
+    if not _CODES:
+        _import_torch()
     if not x.is_cuda:
         raise ValueError(f"{name} must be a CUDA tensor")
     if not x.is_contiguous():
