@@ -255,7 +255,9 @@ class Plan:
 
 # Plans of the functions below that make one a call.  Only plans without a
 # workspace are kept: their execs touch nothing but their arguments and the
-# process-wide tables, so any thread and stream may run one at any time.
+# process-wide tables, so any thread and stream may run one at any time.  The
+# column knobs of the environment are part of what a 2D plan is kept for: of
+# those a plan reads when it is made, no other changes one without a workspace.
 _STATELESS: "OrderedDict[tuple, Plan]" = OrderedDict()
 _STATELESS_MAX = 64
 _stateless_mu = threading.Lock()
@@ -263,6 +265,8 @@ _stateless_mu = threading.Lock()
 
 def _call_plan(*args) -> Plan:
     key = (torch.cuda.current_device(), *args)
+    if args[0] in (KIND_C2C_2D, KIND_R2C_2D):
+        key += (os.environ.get("GFFT_COL_SPLIT"), os.environ.get("GFFT_COL_MAXC"))
     with _stateless_mu:
         p = _STATELESS.get(key)
         if p is not None:
