@@ -178,9 +178,15 @@ def _resolved(x, stream=None):
         return x.resolve_conj().resolve_neg()
 
 
+def _paired(x):
+    """A contiguous x from a boundary of two reals, which the kernels read at a
+    time (a slice of a real tensor may start between two)."""
+    return x.clone() if not x.is_complex() and x.data_ptr() % (2 * x.element_size()) else x
+
+
 def _dense(x):
     """x as the kernels read it: contiguous, its stored values its own."""
-    return _resolved(x).contiguous()
+    return _paired(_resolved(x).contiguous())
 
 
 def _stored(out):
@@ -304,7 +310,7 @@ def _check_cuda_tensor(x, name="x"):
         raise ValueError(f"{name} must be a CUDA tensor")
     if not x.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
-    return _resolved(x)
+    return _paired(_resolved(x))
 
 
 def fft(x, inverse: bool = False, out=None):

@@ -251,6 +251,16 @@ static void check_ptr(const void *ptr, size_t align, const char *name)
     if ((uintptr_t)ptr % align) fail(GFFT_ERR_ALIGN, std::string(name) + " is not aligned to its element type");
 }
 
+// The kernels read and write reals in pairs, so a real array starts on a pair's
+// boundary (rows of more than one real; their distances are even already).
+static size_t real_align(const gfft_desc &d) { return d.n0 > 1 ? 2 * real_bytes(d.dtype) : real_bytes(d.dtype); }
+static void check_real_ptr(const gfft_desc &d, const void *ptr, const char *name)
+{
+    check_ptr(ptr, real_bytes(d.dtype), name);
+    if ((uintptr_t)ptr % real_align(d))
+        fail(GFFT_ERR_ALIGN, std::string(name) + ": real arrays must be aligned to two elements");
+}
+
 // per-call layout (reference-shaped entry points override the plan's)
 struct Layout {
     long long batch, istride, idist, ostride, odist;
@@ -277,8 +287,10 @@ static void exec_body(gfft_plan_s &p, int inverse, void *out, const void *in, co
     const size_t cb = cplx_bytes(d.dtype), rb = real_bytes(d.dtype);
     const bool real_in = (d.kind == GFFT_KIND_R2C && !inverse) || d.kind == GFFT_KIND_R2C_2D;
     const bool real_out = d.kind == GFFT_KIND_R2C && inverse;
-    check_ptr(in, real_in ? rb : cb, "in");
-    check_ptr(out, real_out ? rb : cb, "out");
+    if (real_in) check_real_ptr(d, in, "in");
+    else check_ptr(in, cb, "in");
+    if (real_out) check_real_ptr(d, out, "out");
+    else check_ptr(out, cb, "out");
     switch (d.kind) {
     case GFFT_KIND_C2C:
         if (d.flags & GFFT_FLAG_BITREV_INPUT) {
@@ -409,17 +421,17 @@ static void exec_adjoint(gfft_plan_s &p, int inverse, void *out, const void *in,
         break;
     }
     case GFFT_KIND_R2C: {
-        const size_t cb = cplx_bytes(d.dtype), rb = real_bytes(d.dtype);
+        const size_t cb = cplx_bytes(d.dtype);
         if (!inverse) {
             // adjoint of R2C: C2R of the gradient with interior bins halved
             // (half spectrum) or folded (full spectrum)
             check_ptr(in, cb, "in");
-            check_ptr(out, rb, "out");
+            check_real_ptr(d, out, "out");
             const int w = (d.flags & GFFT_FLAG_HALF_SPECTRUM) ? 1 : 2;
             p.c2r.run(in, out, L.batch, L.odist, L.idist, w, st, scale);
         } else {
             // adjoint of the half-spectrum C2R: R2C with interior bins doubled
-            check_ptr(in, rb, "in");
+            check_real_ptr(d, in, "in");
             check_ptr(out, cb, "out");
             if (!(d.flags & GFFT_FLAG_HALF_SPECTRUM))
                 fail(GFFT_ERR_UNSUPPORTED, "adjoint of the inverse needs a half-spectrum plan");

@@ -36,7 +36,7 @@ typedef enum gfft_status {
     GFFT_ERR_INVALID_SIZE = 1,   /* not a power of two, zero/negative, or above the limit */
     GFFT_ERR_INVALID_VALUE = 2,  /* bad enum, NULL pointer, bad stride */
     GFFT_ERR_ALIAS = 3,          /* out == in where the reference forbids it */
-    GFFT_ERR_ALIGN = 4,          /* pointer not aligned to its element type */
+    GFFT_ERR_ALIGN = 4,          /* pointer not aligned to its element type (real arrays: to two) */
     GFFT_ERR_ARCH = 5,           /* no sm_103 device current */
     GFFT_ERR_CUDA = 6,           /* a CUDA runtime call failed */
     GFFT_ERR_TIMEOUT = 7,        /* a bounded device-side wait gave up */
