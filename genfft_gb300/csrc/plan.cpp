@@ -12,11 +12,17 @@
 //        otherwise                       column + row tile launches per
 //                                        workspace group (tiles*.cuh), the
 //                                        widest TMA-pipelined tile that fits
-//   R2C  n/2 within the fused limit      one fused kernel (real.cu)
-//        fp32 half spectrum above it     tile column pass + row pass with
+//   R2C  n/2 within the fused limit      one fused kernel (real.cu; many
+//                                        fp32 2^14, 2^15: fused_tma.cu)
+//        fp32 half spectrum 2^18 .. 2^22 pipelined column pass + row pass
+//                                        with the DIT fused (real_pipe.cu)
+//        other fp32 half spectra         tile column pass + row pass with
 //                                        the DIT fused (real_4step.cu)
 //        otherwise                       C2C of n/2 + the DIT pass
-//   C2R  n/2 within the fused limit      one fused kernel (c2r.cu)
+//   C2R  n/2 within the fused limit      one fused kernel (c2r.cu; many
+//                                        fp32 2^14, 2^15: fused_tma.cu)
+//        fp32 2^18 .. 2^22               column pass that forms Z' + row
+//                                        pass (real_pipe.cu)
 //        otherwise                       pre-pass + C2C of n/2, inverse
 #include <algorithm>
 #include <cstdint>
@@ -118,9 +124,6 @@ void C2CCore::init(int dtype_, int logn_, long long batch_hint, int path, bool r
     logB = logn - logA;
     const long long N = 1LL << logn;
     const int d = dtype;
-    // inter-pass twiddle W_N^e = tw_hi[e >> lo_bits] * tw_lo[e & (2^lo_bits - 1)]
-    wn_tables(dtype, logn, &lo_bits, &tw_lo, &tw_hi);
-
     // the two-launch tile path: always set up (the persistent kernel needs
     // 16-byte aligned inputs for its tensor copies and uses it otherwise)
     const int maxc = (int)env_ll("GFFT_TILE_MAXC", 16);
@@ -147,7 +150,10 @@ void C2CCore::init(int dtype_, int logn_, long long batch_hint, int path, bool r
     if (!ccol || !crow) fail(GFFT_ERR_UNSUPPORTED, "no tile kernel for this length");
     kcol = tile_find(dtype, vcol, logA, ccol);
     krow = tile_find(dtype, vrow, logB, crow);
+    // inter-pass twiddles: t1 / t2 (tiles_pipe.cuh), or
+    // W_N^e = tw_hi[e >> lo_bits] * tw_lo[e & (2^lo_bits - 1)]
     if (pipe) t12_tables(dtype, logn, kcol, &tw_lo, &tw_hi);
+    else wn_tables(dtype, logn, &lo_bits, &tw_lo, &tw_hi);
     tw_col = tile_table(dtype, kcol, logA, ccol);
     tw_row = tile_table(dtype, krow, logB, crow);
 

@@ -125,7 +125,8 @@ cudaError_t launch_rowpass_dit(const RowDitKernel &k, const void *in, void *out,
 struct R2CCore {
     int dtype = 0, logn = 0, half = 1;
     // 0 n == 1, 1 fused, 2 C2C(n/2) + DIT pass, 3 four-step column pass +
-    // row pass with the DIT fused, 4 one persistent four-step launch whose
+    // row pass with the DIT fused (real_4step.cu; 5 the pipelined passes,
+    // real_pipe.cu), 4 one persistent four-step launch whose
     // row items apply the DIT (3 and 4: half spectrum; other modes as 2)
     int algo = 0;
     const void *tw = nullptr, *dtw = nullptr, *tw_tma = nullptr;

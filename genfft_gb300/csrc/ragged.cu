@@ -1,5 +1,6 @@
 // ragged.cu -- a batch of transforms of uneven power-of-two sizes (fp32,
-// n = 2^0 .. 2^18), packed back to back, in one persistent launch.
+// n = 2^0 .. 2^18), packed back to back: one persistent launch, and before it
+// the launches of the long sizes there is much of.
 //
 // The reference transforms one size per FFT<T> object (fft.h:56-113); a
 // ragged batch there is a host loop over per-size plans.  Here a single
@@ -25,7 +26,10 @@
 // Sizes of 2^16 .. 2^18 with enough transforms take column and row passes of
 // their own before this kernel (ragged_pipe.cu), those of 2^13 and 2^14 the
 // persistent fused kernel (fused_tma.cu), where the input can be read by
-// tensor copies; the batch's other sizes are the list `rest`.
+// tensor copies; the batch's other sizes are the list `rest`.  They run more
+// points a thread than this kernel, so the last bits of a transform of these
+// sizes depend on how many of its size the plan holds and on the input's
+// alignment (not on the schedule).
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -363,8 +363,6 @@ __global__ void __launch_bounds__(C2RColCfg::THREADS, 1)
 
 int realpipe_logl() { return RL; }
 size_t realpipe_twiddle_count() { return RowDitPipeCfg::SP::TW; }
-int realpipe_e() { return RE; }
-int realpipe_g() { return RowDitPipeCfg::SP::G; }
 void realpipe_twiddle_fill(void *buf)
 {
     stockham_fill_twiddles<float, RL, RE>(static_cast<c32 *>(buf), [](long long k, long long M, c32 *w) {

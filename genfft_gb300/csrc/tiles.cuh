@@ -47,8 +47,8 @@ struct ColCfg {
 // tables tw_hi[e >> lo_bits] * tw_lo[e & lo_mask], e = f*i mod N) with
 // f = col (TWM 1: the columns are the second factor) or f = b (TWM 2: the
 // batch index is; one launch covers fewer than 65536 batch items).  TWM 3
-// and 4 are the same two from the tables of tiles_pipe.cuh: tw_lo[f][t] *
-// tw_hi[f][q] for i = t + q G.
+// is TWM 1 from the tables of tiles_pipe.cuh: tw_lo[f][t] * tw_hi[f][q] for
+// i = t + q G.
 // HERM (real 2D output, RealFFT2D::forward, FFTReal.h:90-103): the tile runs
 // over the W/2+1 non-redundant columns (ncols = W/2+1) and also stores the
 // Hermitian mirror X[(L-i) mod L][W-col] = conj X[i][col] for 0 < col < W/2.
@@ -98,13 +98,13 @@ __global__ void __launch_bounds__(ColCfg<T, LOGL, C, E_>::THREADS)
         if (active) {
             cpx<T> *dst = out + b * odist + col + (long long)t * ld_out;
             const long long step = (long long)G * ld_out;
-            const unsigned ecol = TWM == 2 || TWM == 4 ? (unsigned)b : (unsigned)col;
+            const unsigned ecol = TWM == 2 ? (unsigned)b : (unsigned)col;
             cpx<T> w1{(T)0, (T)0};
-            if constexpr (TWM >= 3) w1 = ldg_c(tw_lo + ecol * (unsigned)G + t);
+            if constexpr (TWM == 3) w1 = ldg_c(tw_lo + ecol * (unsigned)G + t);
 #pragma unroll
             for (int q = 0; q < E; q++, dst += step) {
                 cpx<T> val = v[q];
-                if constexpr (TWM >= 3) {
+                if constexpr (TWM == 3) {
                     val = twmul<INV>(val, cmul(w1, ldg_c(tw_hi + ecol * (unsigned)E + q)));
                     if ((q & 7) == 7) asm volatile("" ::: "memory");
                 } else if constexpr (TWM != 0) {

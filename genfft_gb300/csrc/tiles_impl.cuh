@@ -118,7 +118,7 @@ struct PipeReg {
         } else {
             using Cfg = ColCfg<T, LOGL, C, E>;
             using PCfg = PipeCfg<T, LOGL, C, E, NG, NB, LAND_COL>;
-            constexpr int twm = V == TILE_COL_TWP ? 3 : V == TILE_COL_TWB ? 4 : 0;
+            constexpr int twm = V == TILE_COL_TWP ? 3 : 0;
             k.fwd = (const void *)&k_colpass<T, LOGL, C, E, false, twm, false>;
             k.inv = (const void *)&k_colpass<T, LOGL, C, E, true, twm, false>;
             k.threads = Cfg::THREADS;
@@ -130,7 +130,6 @@ struct PipeReg {
             k.tma_boxr = PCfg::BOXR;
             k.tma_rows = PCfg::N;
             k.tma_c = C;
-            k.t12 = twm != 0;
             if constexpr (V == TILE_COL_PLAIN) {
                 using UCfg = PipeCfg<T, LOGL, C, E, NG, NBU, LAND_COLU>;
                 k.tmau_fwd = (const void *)&pipe::k_colpass_tma<T, LOGL, C, E, NG, NBU, false, 0, true>;

@@ -35,8 +35,8 @@
 //   2^21 2925 / 2098   2^22 2851 / 2071   2^23 2788 / 2003   2^24 2651 / 1916
 // and one transform: 2^17 8.9 us / 16.2, 2^20 11.4 / 20.6, 2^24 115 / 146.
 //
-// Inter-pass twiddle W_N^(f k), k = t + q G, f the column (TWM 3) or the
-// batch index (TWM 4): W_N^(f t) * W_N^(G f q) from two tables of directly
+// Inter-pass twiddle W_N^(f k), k = t + q G, f the column (TWM 3):
+// W_N^(f t) * W_N^(G f q) from two tables of directly
 // rounded roots, t1[f][t] (G a row) and t2[f][q] (E a row).  A thread loads
 // one t1 value a tile and the group stages the E x C t2 values it needs,
 // where the hi / lo split costs two scattered loads a point.  (Indexed by the
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU 
     using Cfg = PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU : LAND_COL>;
     static_assert(!U || (TWM == 0 && !AT), "plain columns");
     using SP = typename Cfg::SP;
-    static_assert(sizeof(cpx<T>) == 8 && (TWM == 0 || TWM == 3 || TWM == 4), "fp32; no twiddle, or from t1 / t2");
+    static_assert(sizeof(cpx<T>) == 8 && (TWM == 0 || TWM == 3), "fp32; no twiddle, or from t1 / t2");
     constexpr int E = SP::E, G = SP::G, N = SP::N, GT = Cfg::GT;
     constexpr int W2 = TWM != 0 ? (Cfg::T2 + GT - 1) / GT : 1;  // t2 values a thread stages
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(PipeCfg<T, LOGL, C, E_, NG, NB, U ? LAND_COLU 
         if constexpr (AT) next_off = start_of(i + NB);
         cpx<T> w1{(T)0, (T)0};
         if constexpr (TWM != 0) {
-            const unsigned f = TWM == 3 ? (unsigned)(active ? col : 0) : (unsigned)b;
+            const unsigned f = (unsigned)(active ? col : 0);
             w1 = ldg_c(t1 + f * (unsigned)G + t);
 #pragma unroll
             for (int j = 0; j < W2; j++)

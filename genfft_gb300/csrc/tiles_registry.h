@@ -44,7 +44,6 @@ struct TileKernel {
     size_t tmau_smem = 0;
     int tmau_boxr = 0;
     int e = 0, g = 0;    // points a thread, threads a column (row)
-    bool t12 = false;    // twiddle tables t1 / t2 (tiles_pipe.cuh), not the lo / hi split
     bool tma_row = false;  // a row-pass kernel (for the GFFT_TMA1 knob)
 };
 
