@@ -143,7 +143,7 @@ void fused_twiddle_fill(int dtype, int logn, void *host_buf) { entry_for(dtype, 
 cudaError_t launch_fused_c2c(int dtype, int logn, int inverse, const FusedC2CArgs &a, cudaStream_t st)
 {
     if (a.tw_tma && !a.host && a.istride == 1 && a.ostride == 1 && ((uintptr_t)a.in & 15u) == 0 && a.idist % 2 == 0 &&
-        fused_tma_takes(logn, a.batch))
+        fused_tma_takes(logn, false, a.batch))
         return launch_fused_tma_c2c(logn, inverse, a, st);
     const Entry &e = entry_for(dtype, logn);
     const void *fn = inverse ? e.inv : e.fwd;

@@ -1,27 +1,31 @@
 // fused_tma.cu -- fp32 C2C, R2C and half-spectrum C2R whose complex length is
-// 2^13 or 2^14, dense and on 16-byte boundaries: the arithmetic of k_c2c_fused,
-// k_r2c_fused and k_c2r_fused (32 points a thread), bit for bit, in a persistent
-// kernel that copies a group's next transform in while it stores this one, and
-// keeps the per-thread twiddles in tensor memory.  Not at 2^12: the plain
-// kernels hold 16 points a thread there, and a transform's bits may not depend
-// on how many others stand beside it (host buffers go through in chunks).  With
-// 32 points the plain kernels are 7 - 20 % slower at 2^12 (GB300, us, 16 / 32
-// points: C2C x 152 3.3 / 3.9, x 4096 46.4 / 51.3; R2C x 2000 30.0 / 33.6),
-// which is more than the persistent kernel gains (C2C x 16384 171.4 / 169.4).
+// 2^12 .. 2^14, dense and on 16-byte boundaries: the arithmetic of k_c2c_fused,
+// k_r2c_fused and k_c2r_fused, bit for bit, in a persistent kernel that copies
+// a group's next transform in while it stores this one and keeps the twiddles
+// on chip.  (The same points a thread as the plain kernels, so that a
+// transform's bits do not depend on how many others stand beside it, nor on
+// whether it came from a host buffer, which goes through in chunks.)
 //
-// What bounded the plain kernels at these lengths is the last pass: its table
-// (31 / 32 of N values, 65 KB at 2^13, 129 KB at 2^14) is read once a
-// transform through L1, which the exchange buffers leave no room, so a load a
-// point goes to L2 and is waited for.  Thread t of a group needs the same 31
-// values for every transform (W_N^(t r)), more than its registers hold -- but
-// a persistent CTA has 256 KB of tensor memory beside its registers and
-// shared memory, which tcgen05.st fills once and tcgen05.ld reads back 16
+// What bounded the plain kernels at 2^13 and 2^14 (32 points a thread) is the
+// last pass: its table (31 / 32 of N values, 65 KB at 2^13, 129 KB at 2^14) is
+// read once a transform through L1, which the exchange buffers leave no room,
+// so a load a point goes to L2 and is waited for.  Thread t of a group needs
+// the same 31 values for every transform (W_N^(t r)), more than its registers
+// hold -- but a persistent CTA has 256 KB of tensor memory beside its registers
+// and shared memory, which tcgen05.st fills once and tcgen05.ld reads back 16
 // twiddles at a time.  The real transforms' adjustment twiddles (dit.cuh)
 // lie beside them.  GB300, GB/s, C2C, 1 GB batches: 2^14 5616 with tensor
 // memory, 5110 without it, 3994 the plain kernel; 2^13 6246 / 5044 / 4807.
 // 64 points a thread: 4498 at 2^14, 4506 at 2^13.  Real transforms, n = 2^14 /
 // 2^15, 512 MB - 1 GB: R2C 4896 / 4130 against 4032 / 3453, C2R 5293 / 4945
 // against 3730 / 2982.
+//
+// At 2^12 (16 points a thread) all tables fit shared memory, beside the stages
+// of three transforms (C2C, 80 registers a thread) or four (real, 64).  GB300,
+// us, plain / three / four groups: C2C x 16384 169.7 / 159.6 / 172.7, x 4096
+// 46.3 / 43.9 / 44.7; R2C x 16384 207.2 / 198.4 / 182.4; C2R 212.7 / 207.7 /
+// 180.1.  With 32 points and tensor memory 165.8, 185.9 and 181.3, and the
+// plain kernels are 7 - 20 % slower with 32.
 //
 // Replaces FFT<float>::transform<inv> (fft.h:80-85) and RealFFT<float>::forward
 // (FFTReal.h:186-221) for these lengths.
@@ -42,24 +46,30 @@ using c32 = cpx<float>;
 
 enum FusedKind { FUSED_C2C = 0, FUSED_R2C = 1, FUSED_C2R = 2 };
 
-// NG transforms at a time, a group of N / 32 threads and a stage each
+// NG transforms at a time, a group of N / E threads and a stage each
 template <int LOGN, int NG_, int KIND>
 struct FusedTmaCfg {
-    using SP = StockhamPlan<float, LOGN, 32>;
+    // TM: 32 points a thread, the last pass's and the adjustment's twiddles in
+    // tensor memory; 2^12: the 16 points of the plain kernels, all twiddles in
+    // shared memory
+    static constexpr bool TM = LOGN > 12;
+    using SP = StockhamPlan<float, LOGN, TM ? 32 : 16>;
     static constexpr int N = SP::N, E = SP::E, G = SP::G, NG = NG_, THREADS = G * NG;
     static constexpr int STAGE = (spad_size<float>(N) + 15) / 16 * 16;
-    static constexpr int TWS = SP::twiddle_offset(SP::P - 1);  // every pass but the last: shared memory
+    static constexpr int TWS = TM ? SP::twiddle_offset(SP::P - 1) : SP::TW;  // Stockham twiddles in shared memory
+    static constexpr int DTS = TM || KIND == FUSED_C2C ? 0 : KIND == FUSED_R2C ? N / 2 : N;  // adjustment twiddles there
     // tensor memory: a warp reaches the 32 lanes of its number modulo 4, so
     // warps 4 apart stack their 2 E columns
     // (R2C adds 16 adjustment twiddles a thread, C2R 32)
     static constexpr int WCOLS = KIND == FUSED_C2C ? 2 * E : 4 * E;
     static constexpr int COLS = WCOLS * (THREADS / 128);
-    static constexpr size_t BAR_OFF = ((size_t)NG * STAGE + TWS) * sizeof(c32);
+    static constexpr size_t BAR_OFF = ((size_t)NG * STAGE + (TWS + DTS + 1) / 2 * 2) * sizeof(c32);
     static constexpr size_t SMEM = BAR_OFF + 128;
     static constexpr int PIECE = 4096;  // elements a bulk copy
-    static_assert(E == 32 && SP::P == 3 && THREADS == 512, "three passes, four warps a scheduler");
-    static_assert(COLS <= 512 && (COLS & (COLS - 1)) == 0, "columns");
-    static_assert(2 * SMEM > 228 * 1024, "one CTA an SM: its tensor memory is never waited for by its own grid");
+    static_assert(SP::P == 3 && (TM ? E == 32 && THREADS == 512 : THREADS <= 1024), "three passes");
+    static_assert(!TM || (COLS <= 512 && (COLS & (COLS - 1)) == 0), "columns");
+    static_assert(SMEM <= 227 * 1024 && 2 * SMEM > 228 * 1024,
+                  "one CTA an SM: its tensor memory is never waited for by its own grid");
 };
 
 // 32 consecutive 32-bit columns of this thread's tensor-memory lane
@@ -110,6 +120,8 @@ __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
         fence_barrier_init();
     }
     for (int i = threadIdx.x; i < Cfg::TWS; i += Cfg::THREADS) tws[i] = ldg_c(tw + i);
+    const c32 *const dts = tws + Cfg::TWS;
+    for (int i = threadIdx.x; i < Cfg::DTS; i += Cfg::THREADS) tws[Cfg::TWS + i] = ldg_c(dtw + i);
     // Tensor memory is taken only once every earlier grid is through (a CTA of
     // one that still had its own to allocate would wait for ours while we wait
     // for it), and later grids may come in only once it is taken.
@@ -137,13 +149,15 @@ __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
     };
     if (t == 0) issue(first);
     __syncwarp();
-    if (threadIdx.x < 32) tc::tmem_alloc(tmem_slot, Cfg::COLS);
+    if constexpr (Cfg::TM)
+        if (threadIdx.x < 32) tc::tmem_alloc(tmem_slot, Cfg::COLS);
     __syncthreads();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    tc::fence_after_sync();
-    const int warp = threadIdx.x >> 5;
-    const uint32_t tm = *tmem_slot + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * Cfg::WCOLS;
-    {
+    uint32_t tm = 0;
+    if constexpr (Cfg::TM) {
+        tc::fence_after_sync();
+        const int warp = threadIdx.x >> 5;
+        tm = *tmem_slot + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * Cfg::WCOLS;
         // this thread's last-pass twiddles W_N^(t r) (r = 0: 1, not used),
         // then the adjustment twiddles of bins t + q G
         const c32 *const twl = tw + Cfg::TWS + t;
@@ -178,10 +192,11 @@ __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
 #pragma unroll
             for (int c = 0; c < E / 16; c++) {
                 float r[32];
-                tc::tmem_ld32(tm + (2 + c) * 32, r);
+                if constexpr (Cfg::TM) tc::tmem_ld32(tm + (2 + c) * 32, r);
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
                     const int q = c * 16 + j, k = t + q * G;
+                    const c32 tk = Cfg::TM ? c32{r[2 * j], r[2 * j + 1]} : dts[k];
                     c32 fk = F[k], fp = F[N - k];
                     if (q == 0 && t == 0) {  // bins 0 and N count as real, and whole
                         fk.y = 0.f;
@@ -191,7 +206,7 @@ __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
                         fp = scl(fp, interior);
                     }
                     const c32 sm{fk.x + fp.x, fk.y - fp.y}, df{fp.x - fk.x, -fp.y - fk.y};
-                    const c32 m = cmul(c32{r[2 * j], -r[2 * j + 1]}, df);
+                    const c32 m = cmul(c32{tk.x, -tk.y}, df);
                     v[q] = {sm.x + m.x, sm.y + m.y};
                 }
             }
@@ -216,7 +231,7 @@ __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
 #pragma unroll
             for (int r = 0; r < R0; r++) S[spad<float>((t + m * G) * R0 + r)] = u[r];
         }
-        // pass 1: radix 32, twiddles from shared memory
+        // pass 1: radix E, twiddles from shared memory
         bar_group(bar, G);
 #pragma unroll
         for (int q = 0; q < E; q++) v[q] = S[spad<float>(t + q * G)];
@@ -230,7 +245,7 @@ __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
 #pragma unroll
             for (int r = 0; r < E; r++) S[spad<float>(base + r * R0)] = v[r];
         }
-        // pass 2: radix 32, twiddles from tensor memory
+        // pass 2: radix E, twiddles from tensor memory (2^12: from shared)
         bar_group(bar, G);
 #pragma unroll
         for (int q = 0; q < E; q++) v[q] = S[spad<float>(t + q * G)];
@@ -238,13 +253,19 @@ __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
             stage_read(bar + 1, G, t);
             stage_refill(bar + 1, G, t, true, w + step, issue);
         }
+        if constexpr (Cfg::TM) {
 #pragma unroll
-        for (int c = 0; c < E / 16; c++) {
-            float r[32];
-            tc::tmem_ld32(tm + c * 32, r);
+            for (int c = 0; c < E / 16; c++) {
+                float r[32];
+                tc::tmem_ld32(tm + c * 32, r);
 #pragma unroll
-            for (int j = 0; j < 16; j++)
-                if (c * 16 + j > 0) v[c * 16 + j] = twmul<INV>(v[c * 16 + j], c32{r[2 * j], r[2 * j + 1]});
+                for (int j = 0; j < 16; j++)
+                    if (c * 16 + j > 0) v[c * 16 + j] = twmul<INV>(v[c * 16 + j], c32{r[2 * j], r[2 * j + 1]});
+            }
+        } else {
+            const c32 *const twp = tws + SP::twiddle_offset(SP::P - 1) + t;
+#pragma unroll
+            for (int r = 1; r < E; r++) v[r] = twmul<INV>(v[r], twp[(r - 1) * G]);
         }
         dft<E, INV, float>(v);
         c32 *const dst = out + (AT ? at : (long long)w * odist);
@@ -268,12 +289,12 @@ __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
             stage_read(bar + 1, G, t);
             stage_refill(bar + 1, G, t, true, w + step, issue);
             float r[32];
-            tc::tmem_ld32(tm + 2 * 32, r);
+            if constexpr (Cfg::TM) tc::tmem_ld32(tm + 2 * 32, r);
             const float wt = scale * interior;
 #pragma unroll
             for (int q = 0; q < E / 2; q++) {
                 const int k = t + q * G;
-                const c32 tk{r[2 * q], r[2 * q + 1]};
+                const c32 tk = Cfg::TM ? c32{r[2 * q], r[2 * q + 1]} : dts[k];
                 const bool ends = q == 0 && t == 0;  // bins 0 and N
                 const float f = ends ? scale : wt;
                 stcs_c(dst + k, scl(dit_value(v[q], z[q], tk), f));
@@ -282,30 +303,43 @@ __global__ void __launch_bounds__(FusedTmaCfg<LOGN, NG, KIND>::THREADS, 1)
             if (t == 0) stcs_c(dst + N / 2, scl(dit_value(v[E / 2], v[E / 2], ldg_c(dtw + N / 2)), wt));
         }
     }
-    tc::fence_before_sync();
-    __syncthreads();
-    if (threadIdx.x < 32) tc::tmem_dealloc(*tmem_slot, Cfg::COLS);
+    if constexpr (Cfg::TM) {
+        tc::fence_before_sync();
+        __syncthreads();
+        if (threadIdx.x < 32) tc::tmem_dealloc(*tmem_slot, Cfg::COLS);
+    }
 }
 
 namespace {
 struct Entry {
     const void *fn[6];  // C2C forward and inverse, R2C, C2R, packed C2C forward and inverse
-    int groups;
-    size_t smem[3];     // by kind
+    int groups[3], threads[3];  // by kind
+    size_t smem[3];
 };
-template <int LOGN, int NG>
+// (packed: 2^13 and 2^14 only, see ragged.cu)
+template <int LOGN, int NG, bool INV>
+const void *packed_fn()
+{
+    if constexpr (LOGN > 12) return (const void *)&k_fused_tma<LOGN, NG, FUSED_C2C, INV, true>;
+    else return nullptr;
+}
+// NG groups for C2C, NGR for the real transforms
+template <int LOGN, int NG, int NGR>
 Entry make_entry()
 {
+    using C = FusedTmaCfg<LOGN, NG, FUSED_C2C>;
+    using R = FusedTmaCfg<LOGN, NGR, FUSED_R2C>;
+    using I = FusedTmaCfg<LOGN, NGR, FUSED_C2R>;
     return Entry{{(const void *)&k_fused_tma<LOGN, NG, FUSED_C2C, false>, (const void *)&k_fused_tma<LOGN, NG, FUSED_C2C, true>,
-                  (const void *)&k_fused_tma<LOGN, NG, FUSED_R2C, false>, (const void *)&k_fused_tma<LOGN, NG, FUSED_C2R, true>,
-                  (const void *)&k_fused_tma<LOGN, NG, FUSED_C2C, false, true>, (const void *)&k_fused_tma<LOGN, NG, FUSED_C2C, true, true>},
-                 NG,
-                 {FusedTmaCfg<LOGN, NG, FUSED_C2C>::SMEM, FusedTmaCfg<LOGN, NG, FUSED_R2C>::SMEM,
-                  FusedTmaCfg<LOGN, NG, FUSED_C2R>::SMEM}};
+                  (const void *)&k_fused_tma<LOGN, NGR, FUSED_R2C, false>, (const void *)&k_fused_tma<LOGN, NGR, FUSED_C2R, true>,
+                  packed_fn<LOGN, NG, false>(), packed_fn<LOGN, NG, true>()},
+                 {NG, NGR, NGR},
+                 {C::THREADS, R::THREADS, I::THREADS},
+                 {C::SMEM, R::SMEM, I::SMEM}};
 }
 const Entry &entry(int logn)
 {
-    static const Entry tab[2] = {make_entry<13, 2>(), make_entry<14, 1>()};
+    static const Entry tab[3] = {make_entry<12, 3, 4>(), make_entry<13, 2, 2>(), make_entry<14, 1, 1>()};
     return tab[logn - FUSED_TMA_MIN];
 }
 
@@ -320,36 +354,40 @@ cudaError_t launch(int logn, int kind, int fn_i, const void *in, void *out, long
     int batch = (int)nbatch;
     unsigned *err = device_error_word();
     float scale = (float)sc;
-    const long long grid = std::min<long long>((nbatch + e.groups - 1) / e.groups, sm_count());
+    const long long grid = std::min<long long>((nbatch + e.groups[kind] - 1) / e.groups[kind], sm_count());
     void *args[] = {(void *)&in, (void *)&out, (void *)&batch, (void *)&idist, (void *)&odist, (void *)&tw,
                     (void *)&dtw, (void *)&err, (void *)&scale, (void *)&interior, (void *)&off};
-    return launch_pdl(fn, dim3((unsigned)grid), dim3(512), args, e.smem[kind], st);
+    return launch_pdl(fn, dim3((unsigned)grid), dim3(e.threads[kind]), args, e.smem[kind], st);
 }
 }  // namespace
 
 size_t fused_tma_twiddle_count(int logn)
 {
-    return logn == 13 ? (size_t)StockhamPlan<float, 13, 32>::TW : (size_t)StockhamPlan<float, 14, 32>::TW;
+    return logn == 12 ? (size_t)StockhamPlan<float, 12, 16>::TW
+         : logn == 13 ? (size_t)StockhamPlan<float, 13, 32>::TW : (size_t)StockhamPlan<float, 14, 32>::TW;
 }
 template <int L>
 static void fill(void *buf)
 {
-    stockham_fill_twiddles<float, L, 32>(static_cast<c32 *>(buf), [](long long k, long long M, c32 *w) {
+    stockham_fill_twiddles<float, L, (L > 12 ? 32 : 16)>(static_cast<c32 *>(buf), [](long long k, long long M, c32 *w) {
         forward_root<float>(k, M, &w->x, &w->y);
     });
 }
-void fused_tma_twiddle_fill(int logn, void *buf) { (logn == 13 ? fill<13> : fill<14>)(buf); }
+void fused_tma_twiddle_fill(int logn, void *buf) { (logn == 12 ? fill<12> : logn == 13 ? fill<13> : fill<14>)(buf); }
 
-// The persistent kernels pay for filling tensor memory once a CTA and want
-// transforms to reuse it: more than one wave of the SMs at 2^14, three at 2^13.
-// GB300, us, plain / persistent: C2C 2^14 x 152 12.9 / 13.2, x 304 24.2 / 22.7;
-// 2^13 x 608 21.4 / 21.7, x 1000 33.9 / 32.7; R2C of 2^14 reals x 1000
-// 39.9 / 39.7, x 1501 55.5 / 50.9.
-bool fused_tma_takes(int logn, long long batch)
+// The persistent kernels pay for filling their tables once a CTA and want
+// transforms to reuse them: more than one wave of the SMs at 2^14, three at
+// 2^13, four (C2C) or two (real) at 2^12.  GB300, us, plain / persistent: C2C
+// 2^14 x 152 12.9 / 13.2, x 304 24.2 / 22.7; 2^13 x 608 21.4 / 21.7, x 1000
+// 33.9 / 32.7; 2^12 x 1217 14.3 / 14.5, x 2000 24.6 / 23.8; R2C of 2^14 reals
+// x 1000 39.9 / 39.7, x 1501 55.5 / 50.9; of 2^13 x 608 9.0 / 9.9, x 1217
+// 17.5 / 17.1, x 2000 29.7 / 27.8; C2R of 2^13 x 1217 18.3 / 18.1, x 2000
+// 32.5 / 28.7.
+bool fused_tma_takes(int logn, bool real, long long batch)
 {
     if (logn < FUSED_TMA_MIN || logn > FUSED_TMA_MAX || batch >= (1LL << 30) || !tma_enabled()) return false;
-    const int waves = logn == 14 ? 1 : 3;
-    return batch > waves * entry(logn).groups * (long long)sm_count();
+    const int waves = logn == 14 ? 1 : logn == 13 ? 3 : real ? 2 : 4;
+    return batch > waves * entry(logn).groups[real ? FUSED_R2C : FUSED_C2C] * (long long)sm_count();
 }
 
 cudaError_t launch_fused_tma_c2c(int logn, int inverse, const FusedC2CArgs &a, cudaStream_t st)

@@ -41,12 +41,12 @@ void fused_twiddle_fill(int dtype, int logn, void *host_buf);  // writes that ma
 cudaError_t launch_fused_c2c(int dtype, int logn, int inverse, const FusedC2CArgs &a,
                              cudaStream_t st);
 
-// ---- the persistent versions for fp32, complex lengths 2^13 and 2^14
+// ---- the persistent versions for fp32, complex lengths 2^12 .. 2^14
 // (fused_tma.cu): many transforms of dense, 16-byte aligned input ----------
-constexpr int FUSED_TMA_MIN = 13, FUSED_TMA_MAX = 14;
+constexpr int FUSED_TMA_MIN = 12, FUSED_TMA_MAX = 14;
 size_t fused_tma_twiddle_count(int logn);
 void fused_tma_twiddle_fill(int logn, void *host_buf);
-bool fused_tma_takes(int logn, long long batch);
+bool fused_tma_takes(int logn, bool real, long long batch);
 cudaError_t launch_fused_tma_c2c(int logn, int inverse, const FusedC2CArgs &a, cudaStream_t st);
 // C2C of packed transforms: number w is at element off[w], even
 cudaError_t launch_fused_tma_at(int logn, int inverse, const void *in, void *out, const long long *off, long long count,

@@ -4,7 +4,7 @@
 // Path per size (the defaults, each measured on GB300; the environment
 // knobs read below override them):
 //   C2C  n <= 2^14 (fp32) / 2^13 (fp64)  one fused kernel (c2c_fused.cu; many
-//                                        fp32 2^13, 2^14: fused_tma.cu)
+//                                        fp32 2^12 .. 2^14: fused_tma.cu)
 //        fp32 2^16                       the persistent four-step kernel
 //                                        (fourstep.cuh), one launch a batch
 //        fp32 2^17 .. 2^24               column + row launches of the
@@ -13,14 +13,14 @@
 //                                        workspace group (tiles*.cuh), the
 //                                        widest TMA-pipelined tile that fits
 //   R2C  n/2 within the fused limit      one fused kernel (real.cu; many
-//                                        fp32 2^14, 2^15: fused_tma.cu)
+//                                        fp32 2^13 .. 2^15: fused_tma.cu)
 //        fp32 half spectrum 2^18 .. 2^22 pipelined column pass + row pass
 //                                        with the DIT fused (real_pipe.cu)
 //        other fp32 half spectra         tile column pass + row pass with
 //                                        the DIT fused (real_4step.cu)
 //        otherwise                       C2C of n/2 + the DIT pass
 //   C2R  n/2 within the fused limit      one fused kernel (c2r.cu; many
-//                                        fp32 2^14, 2^15: fused_tma.cu)
+//                                        fp32 2^13 .. 2^15: fused_tma.cu)
 //        fp32 2^18 .. 2^22               column pass that forms Z' + row
 //                                        pass (real_pipe.cu)
 //        otherwise                       pre-pass + C2C of n/2, inverse
@@ -641,7 +641,7 @@ void R2CCore::run(const void *in, void *out, long long batch, long long idist, l
     if (algo == 0) {
         check_cuda(launch_r2c_one(dtype, in, out, batch, idist, odist, st, scale), "launch R2C n=1");
     } else if (algo == 1 && tw_tma && mode != 1 && ((uintptr_t)in & 15u) == 0 && idist % 4 == 0 &&
-               fused_tma_takes(logn - 1, batch)) {
+               fused_tma_takes(logn - 1, true, batch)) {
         check_cuda(launch_fused_tma_r2c(logn - 1, mode == 2, in, out, batch, idist / 2, odist, tw_tma, dtw, st, scale),
                    "launch persistent fused R2C");
     } else if (algo == 1) {
@@ -729,7 +729,7 @@ void C2RCore::run(const void *in, void *out, long long batch, long long idist, l
 {
     if (algo == 0) {
         check_cuda(launch_c2r_one(dtype, in, out, batch, idist, odist, st, scale), "launch C2R n=1");
-    } else if (algo == 1 && tw_tma && wmode != 2 && fused_tma_takes(logn - 1, batch)) {
+    } else if (algo == 1 && tw_tma && wmode != 2 && fused_tma_takes(logn - 1, true, batch)) {
         check_cuda(launch_fused_tma_c2r(logn - 1, wmode == 1, in, out, batch, idist, odist / 2, tw_tma, dtw, st, scale),
                    "launch persistent fused C2R");
     } else if (algo == 1 && !(fold_split && wmode == 2)) {

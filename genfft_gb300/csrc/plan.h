@@ -23,7 +23,7 @@ struct C2CCore {
     int dtype = 0, logn = 0;
     int algo = 0;  // 1 fused, 2 four-step tile launches, 3 persistent four-step, 5 three passes
     const void *tw = nullptr;
-    const void *tw_tma = nullptr;  // algo 1, fp32 2^13 and 2^14: the persistent kernel's (fused_tma.cu)
+    const void *tw_tma = nullptr;  // algo 1, fp32 2^12 .. 2^14: the persistent kernel's (fused_tma.cu)
     // persistent four-step: kernel, ring of `fs_slots` transforms, counters
     const FourStepKernel *fs = nullptr;
     // algo 5: three passes of short tiles (threepass.cu) through `ws`

@@ -507,7 +507,7 @@ static bool ragged_pipe_takes(int logn, long long count)
 // 35 / 69 / 119, fused 32 / 44 / 70; 2^14 34 / 67 / 119, 31 / 49 / 76).
 static bool ragged_fused_takes(int logn, long long count)
 {
-    return (logn == 13 || logn == 14) && (count << logn) >= RAGGED_PIPE_POINTS && fused_tma_takes(logn, count);
+    return (logn == 13 || logn == 14) && (count << logn) >= RAGGED_PIPE_POINTS && fused_tma_takes(logn, false, count);
 }
 
 static bool in_class(const RaggedPlan &p, int logn)

@@ -43,7 +43,7 @@ assert G.device_error() == 0
 
 
 @pytest.mark.parametrize("kind,n0,n1,batch", [
-    ("c2c", 1 << 13, 0, 1000),       # persistent fused kernel
+    ("c2c", 1 << 12, 0, 2000), ("c2c", 1 << 13, 0, 1000),  # persistent fused kernels
     ("c2c", 1 << 15, 0, 2), ("c2c", 1 << 17, 0, 3), ("c2c", 1 << 21, 0, 1),  # column and row passes
     ("r2c", 1 << 15, 0, 400),        # persistent fused kernels
     ("r2c", 1 << 18, 0, 2),          # real passes

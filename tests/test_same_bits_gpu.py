@@ -11,7 +11,7 @@ def same(a, b):
     return torch.equal(torch.view_as_real(a) if a.is_complex() else a, torch.view_as_real(b) if b.is_complex() else b)
 
 
-@pytest.mark.parametrize("logn,batch", [(11, 9001), (12, 9001), (13, 1501), (14, 305)])
+@pytest.mark.parametrize("logn,batch", [(11, 9001), (12, 9001), (12, 1825), (13, 1501), (14, 305)])
 def test_c2c_rows(gfft, logn, batch):
     import torch
     n = 1 << logn
@@ -31,7 +31,7 @@ def test_c2c_rows(gfft, logn, batch):
         assert same(dst, y.cpu())
 
 
-@pytest.mark.parametrize("logn,batch", [(12, 9001), (13, 5001), (14, 1501), (15, 401)])
+@pytest.mark.parametrize("logn,batch", [(12, 9001), (13, 1217), (13, 5001), (14, 1501), (15, 401)])
 def test_real_rows(gfft, logn, batch):
     import torch
     n, m = 1 << logn, (1 << (logn - 1)) + 1
