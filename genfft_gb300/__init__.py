@@ -136,17 +136,19 @@ def _check(status: int) -> None:
 # around it (0.1 us against 2.9), and the dtypes the library takes
 _raw_stream = None
 _CODES: dict = {}
-_COMPLEX: tuple = ()
-_REAL: tuple = ()
+_COMPLEX: dict = {}
+_REAL: dict = {}
+_PAIR: dict = {}  # bytes of two reals
 
 
 def _import_torch():
-    global torch, _raw_stream, _CODES, _COMPLEX, _REAL
+    global torch, _raw_stream, _CODES, _COMPLEX, _REAL, _PAIR
     import torch as module
     _raw_stream = getattr(module._C, "_cuda_getCurrentRawStream", None)
-    _COMPLEX = (module.complex64, module.complex128)
-    _REAL = (module.float32, module.float64)
-    _CODES = {module.complex64: F32, module.float32: F32, module.complex128: F64, module.float64: F64}
+    _COMPLEX = {module.complex64: F32, module.complex128: F64}
+    _REAL = {module.float32: F32, module.float64: F64}
+    _PAIR = {module.float32: 8, module.float64: 16}
+    _CODES = {**_COMPLEX, **_REAL}
     torch = module
     return module
 
@@ -181,7 +183,8 @@ def _resolved(x, stream=None):
 def _paired(x):
     """A contiguous x from a boundary of two reals, which the kernels read at a
     time (a slice of a real tensor may start between two)."""
-    return x.clone() if not x.is_complex() and x.data_ptr() % (2 * x.element_size()) else x
+    size = _PAIR.get(x.dtype)
+    return x if size is None or x.data_ptr() % size == 0 else x.clone()
 
 
 def _dense(x):
@@ -217,7 +220,10 @@ class Plan:
     def exec(self, out, x, inverse: bool = False, stream=None, scale: float = 1.0):
         """Run on torch CUDA tensors (current stream); `scale` multiplies every
         output inside the kernel that writes it."""
-        x, _ = _resolved(x, stream), _stored(out)
+        return self._exec(_stored(out), _resolved(x, stream), inverse, stream, scale)
+
+    def _exec(self, out, x, inverse: bool = False, stream=None, scale: float = 1.0):
+        """exec of tensors whose stored values are their own."""
         if scale == 1.0:
             self.exec_ptr(out.data_ptr(), x.data_ptr(), inverse, _stream_ptr(stream))
         else:
@@ -230,7 +236,9 @@ class Plan:
 
     def adjoint(self, out, g, inverse: bool = False, stream=None, scale: float = 1.0):
         """Adjoint of exec with the same `inverse` and `scale`."""
-        g, _ = _resolved(g, stream), _stored(out)
+        return self._adjoint(_stored(out), _resolved(g, stream), inverse, stream, scale)
+
+    def _adjoint(self, out, g, inverse: bool = False, stream=None, scale: float = 1.0):
         if scale == 1.0:
             self.adjoint_ptr(out.data_ptr(), g.data_ptr(), inverse, _stream_ptr(stream))
         else:
@@ -310,14 +318,17 @@ def _check_cuda_tensor(x, name="x"):
         raise ValueError(f"{name} must be a CUDA tensor")
     if not x.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
-    return _paired(_resolved(x))
+    if x.is_conj() or x.is_neg():
+        x = _resolved(x)
+    return _paired(x) if x.dtype in _PAIR else x
 
 
 def fft(x, inverse: bool = False, out=None):
     """Batched C2C over the last dimension (FFT<T>::transform<inv>, fft.h:80-85).
     The inverse is unscaled."""
     x = _check_cuda_tensor(x)
-    if x.dtype not in _COMPLEX:
+    code = _COMPLEX.get(x.dtype)
+    if code is None:
         raise TypeError("fft expects complex64/complex128")
     n = x.shape[-1]
     batch = x.numel() // n if n else 0
@@ -325,7 +336,7 @@ def fft(x, inverse: bool = False, out=None):
         out = torch.empty_like(x)
     else:
         _stored(out)
-    _check(lib().gfft_fft_transform(_dtype_code(x), n, batch, int(inverse), out.data_ptr(),
+    _check(lib().gfft_fft_transform(code, n, batch, int(inverse), out.data_ptr(),
                                     x.data_ptr(), _stream_ptr()))
     return out
 
@@ -348,7 +359,9 @@ def fft_tc(x, inverse: bool = False, mode: int = MODE_TC_FP16, out=None):
         p = _TC_PLANS[key] = Plan(KIND_C2C, F32, n, 0, batch, mode=mode)
     if out is None:
         out = torch.empty_like(x)
-    return p.exec(out, x, inverse)
+    else:
+        _stored(out)
+    return p._exec(out, x, inverse)
 
 
 def ifft(x, out=None):
@@ -374,15 +387,18 @@ def rfft(x, half: bool = True, out=None):
     """RealFFT<T>::forward over the last dimension (FFTReal.h:204-213):
     n reals -> n/2+1 bins (half) or the full Hermitian n bins."""
     x = _check_cuda_tensor(x)
-    if x.dtype not in _REAL:
+    code = _REAL.get(x.dtype)
+    if code is None:
         raise TypeError("rfft expects float32/float64")
     n = x.shape[-1]
     batch = x.numel() // n
     m = n // 2 + 1 if half else n
     if out is None:
         out = torch.empty(*x.shape[:-1], m, dtype=_cdtype_for_real(x), device=x.device)
-    p = _call_plan(KIND_R2C, _dtype_code(x), n, 0, batch, FLAG_HALF_SPECTRUM if half else 0, 0, n, 0, m)
-    p.exec(out, x)
+    else:
+        _stored(out)
+    p = _call_plan(KIND_R2C, code, n, 0, batch, FLAG_HALF_SPECTRUM if half else 0, 0, n, 0, m)
+    p._exec(out, x)
     return out
 
 
@@ -458,8 +474,10 @@ def fft2(x, inverse: bool = False, out=None):
     batch = x.numel() // (H * W)
     if out is None:
         out = torch.empty_like(x)
+    else:
+        _stored(out)
     p = _call_plan(KIND_C2C_2D, _dtype_code(x), W, H, batch)
-    p.exec(out, x, inverse)
+    p._exec(out, x, inverse)
     return out
 
 
@@ -472,8 +490,10 @@ def rfft2(x, half: bool = False, out=None):
     m = W // 2 + 1 if half else W
     if out is None:
         out = torch.empty(*x.shape[:-1], m, dtype=_cdtype_for_real(x), device=x.device)
+    else:
+        _stored(out)
     p = _call_plan(KIND_R2C_2D, _dtype_code(x), W, H, batch, FLAG_HALF_SPECTRUM if half else 0, W, H * W, m, H * m)
-    p.exec(out, x)
+    p._exec(out, x)
     return out
 
 

@@ -15,7 +15,9 @@ from collections import OrderedDict
 
 import torch
 
-from . import F32, F64, FLAG_HALF_SPECTRUM, KIND_C2C, KIND_R2C, Plan, _dense
+from . import F32, F64, FLAG_HALF_SPECTRUM, KIND_C2C, KIND_R2C, Plan, _dense, _import_torch
+
+_import_torch()
 
 _PLANS: "OrderedDict[tuple, Plan]" = OrderedDict()
 _MAX_PLANS = 64
@@ -47,7 +49,7 @@ class FFTFunction(torch.autograd.Function):
         n = x.shape[-1]
         p = _plan(KIND_C2C, _code(x), n, x.numel() // n)
         y = torch.empty_like(x)
-        p.exec(y, x, inverse)
+        p._exec(y, x, inverse)
         ctx.inverse = inverse
         return y
 
@@ -57,7 +59,7 @@ class FFTFunction(torch.autograd.Function):
         n = g.shape[-1]
         p = _plan(KIND_C2C, _code(g), n, g.numel() // n)
         gx = torch.empty_like(g)
-        p.adjoint(gx, g, ctx.inverse)
+        p._adjoint(gx, g, ctx.inverse)
         return gx, None
 
 
@@ -72,7 +74,7 @@ class RFFTFunction(torch.autograd.Function):
         p = _plan(KIND_R2C, _code(x), n, x.numel() // n, FLAG_HALF_SPECTRUM if half else 0)
         cdt = torch.complex64 if x.dtype == torch.float32 else torch.complex128
         y = torch.empty(*x.shape[:-1], m, dtype=cdt, device=x.device)
-        p.exec(y, x)
+        p._exec(y, x)
         ctx.half, ctx.n = half, n
         return y
 
@@ -83,7 +85,7 @@ class RFFTFunction(torch.autograd.Function):
         p = _plan(KIND_R2C, _code(g), n, g.numel() // g.shape[-1], FLAG_HALF_SPECTRUM if ctx.half else 0)
         rdt = torch.float32 if g.dtype == torch.complex64 else torch.float64
         gx = torch.empty(*g.shape[:-1], n, dtype=rdt, device=g.device)
-        p.adjoint(gx, g, False)
+        p._adjoint(gx, g, False)
         return gx, None
 
 
@@ -96,7 +98,7 @@ class IRFFTFunction(torch.autograd.Function):
         p = _plan(KIND_R2C, _code(y), n, y.numel() // y.shape[-1], FLAG_HALF_SPECTRUM)
         rdt = torch.float32 if y.dtype == torch.complex64 else torch.float64
         x = torch.empty(*y.shape[:-1], n, dtype=rdt, device=y.device)
-        p.exec(x, y, True)
+        p._exec(x, y, True)
         ctx.n = n
         return x
 
@@ -107,7 +109,7 @@ class IRFFTFunction(torch.autograd.Function):
         p = _plan(KIND_R2C, _code(g), n, g.numel() // n, FLAG_HALF_SPECTRUM)
         cdt = torch.complex64 if g.dtype == torch.float32 else torch.complex128
         gy = torch.empty(*g.shape[:-1], n // 2 + 1, dtype=cdt, device=g.device)
-        p.adjoint(gy, g, True)
+        p._adjoint(gy, g, True)
         return gy, None
 
 

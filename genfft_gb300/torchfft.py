@@ -27,7 +27,9 @@ import torch
 import torch.autograd.forward_ad as _forward_ad
 
 from . import (F32, F64, FLAG_HALF_SPECTRUM, KIND_C2C, KIND_C2C_2D, KIND_R2C, KIND_R2C_2D, KIND_VERT,
-               Plan, _dense)
+               Plan, _dense, _import_torch)
+
+_import_torch()
 
 __all__ = ["fft", "ifft", "rfft", "irfft", "fft2", "ifft2", "rfft2", "irfft2", "norm_scale"]
 
@@ -110,14 +112,14 @@ def _c2c(x, inverse: bool, scale: float):
     x = _dense(x)
     n = x.shape[-1]
     p = _plan(KIND_C2C, _code(x), n, 0, x.numel() // n)
-    return p.exec(torch.empty_like(x), x, inverse, scale=scale)
+    return p._exec(torch.empty_like(x), x, inverse, scale=scale)
 
 
 def _c2c2d(x, inverse: bool, scale: float):
     x = _dense(x)
     h, w = x.shape[-2], x.shape[-1]
     p = _plan(KIND_C2C_2D, _code(x), w, h, x.numel() // (h * w))
-    return p.exec(torch.empty_like(x), x, inverse, scale=scale)
+    return p._exec(torch.empty_like(x), x, inverse, scale=scale)
 
 
 def _r2c(x, scale: float):
@@ -126,7 +128,7 @@ def _r2c(x, scale: float):
     p = _plan(KIND_R2C, _code(x), n, 0, x.numel() // n, FLAG_HALF_SPECTRUM)
     cdt = torch.complex128 if x.dtype == torch.float64 else torch.complex64
     y = torch.empty(*x.shape[:-1], n // 2 + 1, dtype=cdt, device=x.device)
-    return p.exec(y, x, False, scale=scale)
+    return p._exec(y, x, False, scale=scale)
 
 
 def _c2r(y, n: int, scale: float):
@@ -134,7 +136,7 @@ def _c2r(y, n: int, scale: float):
     p = _plan(KIND_R2C, _code(y), n, 0, y.numel() // y.shape[-1], FLAG_HALF_SPECTRUM)
     rdt = torch.float64 if y.dtype == torch.complex128 else torch.float32
     x = torch.empty(*y.shape[:-1], n, dtype=rdt, device=y.device)
-    return p.exec(x, y, True, scale=scale)
+    return p._exec(x, y, True, scale=scale)
 
 
 class _C2C(torch.autograd.Function):
@@ -173,7 +175,7 @@ class _R2C(torch.autograd.Function):
         p = _plan(KIND_R2C, _code(g), n, 0, g.numel() // g.shape[-1], FLAG_HALF_SPECTRUM)
         rdt = torch.float64 if g.dtype == torch.complex128 else torch.float32
         gx = torch.empty(*g.shape[:-1], n, dtype=rdt, device=g.device)
-        return p.adjoint(gx, g, False, scale=ctx.scale), None
+        return p._adjoint(gx, g, False, scale=ctx.scale), None
 
 
 class _C2R(torch.autograd.Function):
@@ -189,7 +191,7 @@ class _C2R(torch.autograd.Function):
         p = _plan(KIND_R2C, _code(g), n, 0, g.numel() // n, FLAG_HALF_SPECTRUM)
         cdt = torch.complex128 if g.dtype == torch.float64 else torch.complex64
         gy = torch.empty(*g.shape[:-1], n // 2 + 1, dtype=cdt, device=g.device)
-        return p.adjoint(gy, g, True, scale=ctx.scale), None, None
+        return p._adjoint(gy, g, True, scale=ctx.scale), None, None
 
 
 def _plain(x) -> bool:
@@ -321,7 +323,7 @@ def rfft2(input, s=None, dim=(-2, -1), norm=None):
     p = _plan(KIND_R2C_2D, _code(x), w, h, batch, FLAG_HALF_SPECTRUM)
     cdt = torch.complex128 if x.dtype == torch.float64 else torch.complex64
     y = torch.empty(*x.shape[:-1], w // 2 + 1, dtype=cdt, device=x.device)
-    p.exec(y, x, False, scale=norm_scale(norm, h * w, False))
+    p._exec(y, x, False, scale=norm_scale(norm, h * w, False))
     return _back2(y, d0, d1)
 
 
@@ -343,9 +345,9 @@ def irfft2(input, s=None, dim=(-2, -1), norm=None):
     batch = y.numel() // (h * m)
     cols = _plan(KIND_VERT, _code(y), h, m, batch)
     t = torch.empty_like(y)
-    cols.exec(t, y, True)
+    cols._exec(t, y, True)
     rows = _plan(KIND_R2C, _code(y), w, 0, batch * h, FLAG_HALF_SPECTRUM)
     rdt = torch.float64 if y.dtype == torch.complex128 else torch.float32
     x = torch.empty(*y.shape[:-1], w, dtype=rdt, device=y.device)
-    rows.exec(x, t, True, scale=norm_scale(norm, h * w, True))
+    rows._exec(x, t, True, scale=norm_scale(norm, h * w, True))
     return _back2(x, d0, d1)
