@@ -132,9 +132,10 @@ def _check(status: int) -> None:
         raise GFFTError(status, msg.decode() if msg else "")
 
 
-# set by _import_torch: the current stream's handle without a Stream object
-# around it (0.1 us against 2.9), and the dtypes the library takes
-_raw_stream = None
+# set by _import_torch: the current device, its current stream's handle
+# without a Stream object around it (0.1 us against 2.9), and the dtypes the
+# library takes
+_raw_device = _raw_stream = None
 _CODES: dict = {}
 _COMPLEX: dict = {}
 _REAL: dict = {}
@@ -142,9 +143,10 @@ _PAIR: dict = {}  # bytes of two reals
 
 
 def _import_torch():
-    global torch, _raw_stream, _CODES, _COMPLEX, _REAL, _PAIR
+    global torch, _raw_device, _raw_stream, _CODES, _COMPLEX, _REAL, _PAIR
     import torch as module
     _raw_stream = getattr(module._C, "_cuda_getCurrentRawStream", None)
+    _raw_device = getattr(module._C, "_cuda_getDevice", None) or module.cuda.current_device
     _COMPLEX = {module.complex64: F32, module.complex128: F64}
     _REAL = {module.float32: F32, module.float64: F64}
     _PAIR = {module.float32: 8, module.float64: 16}
@@ -157,7 +159,7 @@ def _stream_ptr(stream=None) -> int:
     if stream is not None:
         return stream.cuda_stream
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_raw_device())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -215,7 +217,9 @@ class Plan:
         return self._h
 
     def exec_ptr(self, out_ptr: int, in_ptr: int, inverse: bool = False, stream_ptr: int = 0):
-        _check(lib().gfft_exec(self._h, int(inverse), out_ptr, in_ptr, stream_ptr))
+        status = (_lib or lib()).gfft_exec(self._h, int(inverse), out_ptr, in_ptr, stream_ptr)
+        if status:
+            _check(status)
 
     def exec(self, out, x, inverse: bool = False, stream=None, scale: float = 1.0):
         """Run on torch CUDA tensors (current stream); `scale` multiplies every
@@ -275,12 +279,17 @@ class Plan:
 _STATELESS: "OrderedDict[tuple, Plan]" = OrderedDict()
 _STATELESS_MAX = 64
 _stateless_mu = threading.Lock()
+# os.environ.get, or the dict behind it (0.1 us against 0.8 for a name that is
+# not there)
+_ENV = getattr(os.environ, "_data", os.environ).get
+_COL_SPLIT, _COL_MAXC = (os.environ.encodekey(k) if hasattr(os.environ, "_data") else k
+                         for k in ("GFFT_COL_SPLIT", "GFFT_COL_MAXC"))
 
 
 def _call_plan(*args) -> Plan:
     key = (torch.cuda.current_device(), *args)
     if args[0] in (KIND_C2C_2D, KIND_R2C_2D):
-        key += (os.environ.get("GFFT_COL_SPLIT"), os.environ.get("GFFT_COL_MAXC"))
+        key += (_ENV(_COL_SPLIT), _ENV(_COL_MAXC))
     with _stateless_mu:
         p = _STATELESS.get(key)
         if p is not None:
@@ -336,8 +345,10 @@ def fft(x, inverse: bool = False, out=None):
         out = torch.empty_like(x)
     else:
         _stored(out)
-    _check(lib().gfft_fft_transform(code, n, batch, int(inverse), out.data_ptr(),
-                                    x.data_ptr(), _stream_ptr()))
+    status = (_lib or lib()).gfft_fft_transform(code, n, batch, int(inverse), out.data_ptr(), x.data_ptr(),
+                                                _stream_ptr())
+    if status:
+        _check(status)
     return out
 
 
