@@ -421,30 +421,52 @@ def run_reference(args):
     return 0
 
 
-def kernel_name(G, kind, dtype, n0, mode=0, launches=1):
-    """The kernels of one exec of the workload (`launches`: the plan's
-    launch count for the batch; the four-step path is one persistent
-    launch, column + row tile launches per workspace group, or, for fp32
-    2^21 .. 2^24, three short-tile passes per group)."""
+# batches above which fp32 transforms of complex length 2^l take the persistent
+# fused kernel, in waves of the SMs x transforms a CTA holds: C2C, real
+# (fused_tma_takes in csrc/fused_tma.cu)
+FUSED_TMA_WAVES = {12: (4 * 3, 2 * 4), 13: (3 * 2, 3 * 2), 14: (1, 1)}
+
+
+def fused_name(plain, dtype, log_complex, real, rows, sms):
+    if dtype == "f32" and log_complex in FUSED_TMA_WAVES and sms and \
+            rows > FUSED_TMA_WAVES[log_complex][1 if real else 0] * sms:
+        return "k_fused_tma"
+    return plain
+
+
+def kernel_name(G, kind, dtype, n0, mode=0, launches=1, batch=0, n1=0, sms=0, three_pass=None):
+    """The kernels of one exec of the workload (`launches`: the plan's launch
+    count for the batch; `sms`: the device's SMs, 0 where the batch is not to
+    be looked at; `three_pass`: whether GFFT_3PASS asks for three passes, by
+    default read off the launch count)."""
     if mode:
         return "k_tc"
     fused = n0 <= G.max_fused_size(G.F32 if dtype == "f32" else G.F64)
+    half_fused = n0 // 2 <= G.max_fused_size(G.F32 if dtype == "f32" else G.F64)
+    logn = n0.bit_length() - 1
+    pipelined = dtype == "f32" and 18 <= logn <= 22  # half spectra, csrc/real_pipe.cu
     if kind == "c2c":
         if fused:
-            return "k_c2c_fused"
+            return fused_name("k_c2c_fused", dtype, logn, False, batch, sms)
         if launches == 1:
             return "k_fourstep"
-        if launches % 3 == 0 and dtype == "f32" and n0 >= (1 << 21):
+        if three_pass is None:
+            three_pass = launches % 3 == 0 and n0 >= (1 << 21)
+        if three_pass and dtype == "f32":
             return "k3_col (two column passes) + k3_row"
         return "k_colpass_tma + k_rowpass_tma"
     if kind == "c2r":
-        return "k_c2r_fused" if n0 // 2 <= G.max_fused_size(G.F32) else "C2R pre-pass + four-step inverse"
+        if half_fused:
+            return fused_name("k_c2r_fused", dtype, logn - 1, True, batch, sms)
+        return "k_c2rcol_pipe + k_rowpass_tma" if pipelined else "C2R pre-pass + four-step inverse"
     if kind == "r2c":
-        return "k_r2c_fused" if n0 // 2 <= G.max_fused_size(G.F32) else "k_colpass_tma + k_rowpass_dit"
+        if half_fused:
+            return fused_name("k_r2c_fused", dtype, logn - 1, True, batch, sms)
+        return "k_colpass_tma + k_rowdit_pipe" if pipelined else "k_colpass_tma + k_rowpass_dit"
     if kind == "c2d":
-        return "k_c2c_fused (rows) + k_colpass (columns)"
+        return fused_name("k_c2c_fused", dtype, logn, False, batch * n1, sms) + " (rows) + k_colpass_tma (columns)"
     if kind == "r2d":
-        return "k_r2c_fused (rows) + k_colpass Hermitian (columns)"
+        return fused_name("k_r2c_fused", dtype, logn - 1, True, batch * n1, sms) + " (rows) + k_colpass_tma (columns)"
     return "plan kernels"
 
 
@@ -500,7 +522,7 @@ def ragged_sizes(count, seed=20240):
 
 
 def run_ragged(args):
-    """Ragged batch: one persistent graph-captured launch per exec; also the
+    """Ragged batch: one graph launch per exec (`launches` kernels); also the
     same transforms as one uniform C2C launch per size class (the uniform
     time per byte) for comparison."""
     import numpy as np
@@ -610,7 +632,8 @@ def run_ragged(args):
                          "traffic": traffic_from_profile(args.workload),
                          "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)" if peak_src == "measured"
                          else "fallback 6800 GB/s",
-                         "kernel": "k_colpass_tma, k_rowpass_tma, k_ragged" if plan.launches > 1 else "k_ragged",
+                         "kernel": "k_colpass_tma, k_rowpass_tma (2^16 .. 2^18), k_fused_tma (2^13, 2^14), k_ragged"
+                         if plan.launches > 1 else "k_ragged",
                          "launches_per_exec": plan.launches, "avg_exec_ms": round(exec_ms, 5),
                          "algorithmic_bytes_per_exec": bytes_exec},
             "e2e": {"value": round(e2e_gbs, 2), "unit": "GB/s", "h2d_bytes_per_step": 2 * 8 * plan.elements,
@@ -705,7 +728,9 @@ def companion(G, torch, name, steps, warmup, dev):
                         "frac": round(achieved / peak, 4), "traffic": traffic_from_profile(name),
                         "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)" if peak_src == "measured"
                         else "fallback 6800 GB/s",
-                        "kernel": kernel_name(G, kind, dtype, n0, mode, launches_per_exec),
+                        "kernel": kernel_name(G, kind, dtype, n0, mode, launches_per_exec, batch, n1,
+                                              torch.cuda.get_device_properties(0).multi_processor_count,
+                                              os.environ.get("GFFT_3PASS", "0") not in ("", "0")),
                         "launches_per_exec": launches_per_exec, "avg_exec_ms": round(avg_exec_ms, 5),
                         "duration_source": "the timed region / (steps x execs), gaps between launches included",
                         "algorithmic_bytes_per_exec": batch * per_transform},
@@ -850,7 +875,9 @@ def run_ours(args):
                          "frac": round(achieved / peak, 4), "traffic": traffic,
                          "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)" if peak_src == "measured"
                          else "fallback 6800 GB/s",
-                         "kernel": kernel_name(G, kind, dtype, n0, mode, launches_per_exec),
+                         "kernel": kernel_name(G, kind, dtype, n0, mode, launches_per_exec, batch, n1,
+                                              torch.cuda.get_device_properties(0).multi_processor_count,
+                                              os.environ.get("GFFT_3PASS", "0") not in ("", "0")),
                          "launches_per_exec": launches_per_exec, "avg_exec_ms": round(avg_exec_ms, 5),
                          "avg_launch_ms": round(avg_launch_ms, 5),
                          "duration_source": "the timed region / (steps x execs), gaps between launches included",
