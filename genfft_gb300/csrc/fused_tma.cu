@@ -14,8 +14,9 @@
 // hold -- but a persistent CTA has 256 KB of tensor memory beside its registers
 // and shared memory, which tcgen05.st fills once and tcgen05.ld reads back 16
 // twiddles at a time.  The real transforms' adjustment twiddles (dit.cuh)
-// lie beside them.  GB300, GB/s, C2C, 1 GB batches: 2^14 5616 with tensor
-// memory, 5110 without it, 3994 the plain kernel; 2^13 6246 / 5044 / 4807.
+// lie beside them.  GB300, GB/s, C2C, 1 GB batches: 2^14 5430 - 5660 from run
+// to run with tensor memory, 5110 without it, 3994 the plain kernel; 2^13 6120 -
+// 6250 / 5044 / 4807.
 // 64 points a thread: 4498 at 2^14, 4506 at 2^13.  Real transforms, n = 2^14 /
 // 2^15, 512 MB - 1 GB: R2C 4896 / 4130 against 4032 / 3453, C2R 5293 / 4945
 // against 3730 / 2982.

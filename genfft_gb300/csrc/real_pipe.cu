@@ -22,9 +22,9 @@
 // read and one write of the reals, against the 16-point passes before (column
 // tiles + row pass with the DIT; pre-pass + C2C of n/2):
 //            forward                     inverse
-//   2^18     2^18 x 64 2483 / 1896       2051 / 1454
-//   2^20     x 64      2299 / 1712       2248 / 1483
-//   2^20     x 1       10.4 us / 19.2    11.3 us / 24.6
+//   2^18     x 64      2488 / 1896       2276 / 1454
+//   2^20     x 64      2370 / 1712       2534 / 1483
+//   2^20     x 1       10.1 us / 19.2    11.2 us / 24.6
 // Its partial 64-byte runs (the half spectrum has H + 1 bins, so every other
 // transform starts 8 bytes off a boundary) cost 1.4x the L2 write sectors.
 #include <algorithm>

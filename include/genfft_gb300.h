@@ -102,7 +102,12 @@ gfft_status gfft_plan_destroy(gfft_plan plan);
  * For GFFT_KIND_R2C plans the inverse is the half-spectrum inverse (C2R):
  * bins in the plan's output layout -> reals in its input layout, unscaled,
  * imaginary parts of the DC and Nyquist bins ignored (no counterpart in the
- * reference, whose RealFFT has no inverse, FFTReal.h:127-130). */
+ * reference, whose RealFFT has no inverse, FFTReal.h:127-130).
+ * `in` and `out` are aligned to their elements, real arrays to two of them
+ * (rows of one real excepted).  Kernels with TMA copies load whole 16-byte
+ * granules: up to 8 bytes before and after an input that starts or ends inside
+ * one are read too, and not used.  A transform's bits do not depend on the
+ * batch or the columns it stands beside, nor on the alignment. */
 gfft_status gfft_exec(gfft_plan plan, int inverse, void *out, const void *in, void *stream);
 /* gfft_exec with every output multiplied by `scale` inside the kernel that
  * writes it (no extra pass): the norm= factors of torch.fft-style APIs
@@ -214,7 +219,8 @@ gfft_status gfft_separate_2x_real_fft(int dtype, int n, void *out1, void *out2, 
  * a synchronous table upload): make it before any stream capture.  All calls
  * share the scratch, so calls that can overlap on the GPU race and must be
  * serialised by the caller.  Sizes outside 2^15 .. 2^22 and fp64 are
- * rejected.  Same results as gfft_fft_transform. */
+ * rejected.  Same results as gfft_fft_transform, to rounding (it keeps the
+ * two-launch tiles at every length). */
 gfft_status gfft_fft_transform_noalloc(int dtype, int n, long long batch, int inverse, void *out,
                                        const void *in, void *stream);
 
@@ -222,11 +228,14 @@ gfft_status gfft_fft_transform_noalloc(int dtype, int n, long long batch, int in
  * size per FFT<T> object, fft.h:56-113) ----------------------------------
  * `count` fp32 C2C transforms of power-of-two sizes 1 .. 2^18 packed back to
  * back (transform i starts at the sum of the earlier sizes).  One exec is
- * one CUDA-graph replay of a single persistent kernel; the graph is
+ * one CUDA-graph replay (gfft_ragged_launches kernels); the graph is
  * captured on the first exec with a given (in, out, direction).  The plan
  * owns scratch for its transforms above 2^12 points and a work counter:
  * execs of one plan must be ordered by the caller (one stream, or events);
- * use one plan per stream to run ragged batches concurrently. */
+ * use one plan per stream to run ragged batches concurrently.  Sizes of
+ * 2^13, 2^14 and 2^16 .. 2^18 run other kernels where the plan holds many of
+ * them and `in` is 16-byte aligned: there the last bits of a transform depend
+ * on the plan's other sizes and on the alignment, within the same bounds. */
 typedef struct gfft_ragged_s *gfft_ragged;
 gfft_status gfft_ragged_create(gfft_ragged *plan, int dtype, const long long *sizes, long long count);
 gfft_status gfft_ragged_destroy(gfft_ragged plan);
