@@ -91,3 +91,51 @@ def test_batches_of_real_images(gfft, h, w, batch):
     assert same(half, full[..., :w // 2 + 1].contiguous())
     for b in (0, batch - 1):
         assert same(gfft.rfft2(x[b], half=True), half[b]) and same(gfft.rfft2(x[b]), full[b])
+
+
+@pytest.mark.parametrize("dtype,logn,batch", [("f32", 15, 7), ("f32", 16, 9), ("f32", 17, 5), ("f32", 18, 80), ("f32", 20, 5),
+                                              ("f32", 22, 3), ("f32", 24, 2), ("f64", 13, 30), ("f64", 14, 9),
+                                              ("f64", 16, 5), ("f64", 20, 2)])
+def test_multipass_rows(gfft, dtype, logn, batch):
+    import torch
+    n, code = 1 << logn, gfft.F32 if dtype == "f32" else gfft.F64
+    cplx = torch.complex64 if dtype == "f32" else torch.complex128
+    x = torch.randn(batch, n, dtype=cplx, device="cuda")
+    p, one = gfft.Plan(gfft.KIND_C2C, code, n, 0, batch), gfft.Plan(gfft.KIND_C2C, code, n, 0, 1)
+    for inv in (False, True):
+        y = p.exec(torch.empty_like(x), x, inv)
+        for k in (0, batch - 1):
+            assert same(one.exec(torch.empty_like(x[:1]), x[k:k + 1].clone(), inv), y[k:k + 1])
+        if dtype == "f32":
+            odd = torch.empty(batch * n + 1, dtype=cplx, device="cuda")[1:].view(batch, n)
+            odd.copy_(x)  # off a 16-byte boundary
+            assert same(p.exec(torch.empty_like(x), odd, inv), y)
+
+
+@pytest.mark.parametrize("logn,batch", [(16, 5), (17, 4), (18, 70), (19, 3), (20, 3), (22, 2), (23, 2)])
+def test_multipass_real_rows(gfft, logn, batch):
+    import torch
+    n, m = 1 << logn, (1 << (logn - 1)) + 1
+    x = torch.randn(batch, n, device="cuda")
+    f = torch.randn(batch, m, dtype=torch.complex64, device="cuda")
+    p = gfft.Plan(gfft.KIND_R2C, gfft.F32, n, 0, batch, gfft.FLAG_HALF_SPECTRUM)
+    one = gfft.Plan(gfft.KIND_R2C, gfft.F32, n, 0, 1, gfft.FLAG_HALF_SPECTRUM)
+    y, z = torch.empty_like(f), torch.empty_like(x)
+    for call, src, inv, out in (("exec", x, False, y), ("exec", f, True, z), ("adjoint", f, False, z),
+                                ("adjoint", x, True, y)):
+        getattr(p, call)(out, src, inv)
+        for k in (0, batch - 1):
+            assert same(getattr(one, call)(torch.empty_like(out[:1]), src[k:k + 1].clone(), inv), out[k:k + 1]), (call, inv)
+        pad = 2 if src is x else 1
+        odd = torch.empty(src.numel() + pad, dtype=src.dtype, device="cuda")[pad:].view(src.shape)
+        odd.copy_(src)
+        assert same(getattr(p, call)(torch.empty_like(out), odd, inv), out), (call, inv)
+
+
+@pytest.mark.parametrize("h,w,batch", [(64, 4096, 40), (1024, 512, 9), (2048, 2048, 3), (32, 1 << 16, 3)])
+def test_batches_of_images(gfft, h, w, batch):
+    import torch
+    x = torch.randn(batch, h, w, dtype=torch.complex64, device="cuda")
+    y = gfft.fft2(x)
+    for b in (0, batch - 1):
+        assert same(gfft.fft2(x[b].clone()), y[b])
