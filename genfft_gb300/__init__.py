@@ -185,13 +185,15 @@ def _resolved(x, stream=None):
 def _paired(x):
     """A contiguous x from a boundary of two reals, which the kernels read at a
     time (a slice of a real tensor may start between two)."""
-    size = _PAIR.get(x.dtype)
-    return x if size is None or x.data_ptr() % size == 0 else x.clone()
+    return x.clone() if x.data_ptr() % _PAIR[x.dtype] else x
 
 
 def _dense(x):
     """x as the kernels read it: contiguous, its stored values its own."""
-    return _paired(_resolved(x).contiguous())
+    if x.is_conj() or x.is_neg():
+        x = _resolved(x)
+    x = x.contiguous()
+    return _paired(x) if x.dtype in _PAIR else x
 
 
 def _stored(out):
@@ -217,22 +219,26 @@ class Plan:
         return self._h
 
     def exec_ptr(self, out_ptr: int, in_ptr: int, inverse: bool = False, stream_ptr: int = 0):
-        status = (_lib or lib()).gfft_exec(self._h, int(inverse), out_ptr, in_ptr, stream_ptr)
-        if status:
-            _check(status)
+        _check(lib().gfft_exec(self._h, int(inverse), out_ptr, in_ptr, stream_ptr))
 
     def exec(self, out, x, inverse: bool = False, stream=None, scale: float = 1.0):
         """Run on torch CUDA tensors (current stream); `scale` multiplies every
         output inside the kernel that writes it."""
-        return self._exec(_stored(out), _resolved(x, stream), inverse, stream, scale)
+        if out.is_conj() or out.is_neg():
+            _stored(out)
+        if x.is_conj() or x.is_neg():
+            x = _resolved(x, stream)
+        return self._exec(out, x, inverse, stream, scale)
 
     def _exec(self, out, x, inverse: bool = False, stream=None, scale: float = 1.0):
         """exec of tensors whose stored values are their own."""
+        st = _raw_stream(_raw_device()) if stream is None and _raw_stream is not None else _stream_ptr(stream)
         if scale == 1.0:
-            self.exec_ptr(out.data_ptr(), x.data_ptr(), inverse, _stream_ptr(stream))
+            status = _lib.gfft_exec(self._h, 1 if inverse else 0, out.data_ptr(), x.data_ptr(), st)
         else:
-            _check(lib().gfft_exec_scaled(self._h, int(inverse), float(scale), out.data_ptr(), x.data_ptr(),
-                                          _stream_ptr(stream)))
+            status = _lib.gfft_exec_scaled(self._h, 1 if inverse else 0, float(scale), out.data_ptr(), x.data_ptr(), st)
+        if status:
+            _check(status)
         return out
 
     def adjoint_ptr(self, out_ptr: int, in_ptr: int, inverse: bool = False, stream_ptr: int = 0):
@@ -335,18 +341,20 @@ def _check_cuda_tensor(x, name="x"):
 def fft(x, inverse: bool = False, out=None):
     """Batched C2C over the last dimension (FFT<T>::transform<inv>, fft.h:80-85).
     The inverse is unscaled."""
-    x = _check_cuda_tensor(x)
     code = _COMPLEX.get(x.dtype)
-    if code is None:
-        raise TypeError("fft expects complex64/complex128")
+    if code is None or not x.is_cuda or not x.is_contiguous() or x.is_conj() or x.is_neg():
+        x = _check_cuda_tensor(x)
+        code = _COMPLEX.get(x.dtype)
+        if code is None:
+            raise TypeError("fft expects complex64/complex128")
     n = x.shape[-1]
     batch = x.numel() // n if n else 0
     if out is None:
         out = torch.empty_like(x)
     else:
         _stored(out)
-    status = (_lib or lib()).gfft_fft_transform(code, n, batch, int(inverse), out.data_ptr(), x.data_ptr(),
-                                                _stream_ptr())
+    status = (_lib or lib()).gfft_fft_transform(code, n, batch, 1 if inverse else 0, out.data_ptr(), x.data_ptr(),
+                                                _raw_stream(_raw_device()) if _raw_stream else _stream_ptr())
     if status:
         _check(status)
     return out
